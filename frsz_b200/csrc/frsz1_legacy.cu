@@ -14,10 +14,10 @@
 // round-to-nearest operations (no contraction), as in the reference's build.
 //
 // compress is elementwise: a thread takes 8 consecutive values, its left
-// neighbour's quantized value by a shuffle, and writes 16 bytes.  decompress runs one thread per block of
-// 256 values (the sum is sequential and rounds at every step); 64 blocks per
-// CTA go out through shared memory 16 values at a time, so the stores are
-// coalesced.
+// neighbour's quantized value by a shuffle, and writes 16 bytes.  decompress
+// runs one thread per block of 256 values (the sum is sequential and rounds at
+// every step); codes and values go through shared memory, so the global
+// accesses are coalesced.
 #include "frsz2_fast.cuh"
 #include "frsz2_launch.hpp"
 
@@ -221,6 +221,173 @@ __device__ __forceinline__ T legacy_step(std::int16_t q, double ebx2, T prev)
     return t;
 }
 
+// One block of 256 values per thread; a CTA is one warp, so 32 blocks.  The
+// codes come in stages through a pair of shared-memory buffers (asynchronous
+// 16-byte copies, the next stage in flight while the current one is summed) and
+// the values leave 64 per block at a time through a third; rows are an odd
+// multiple of 16 bytes apart, which keeps each thread's 16-byte accesses to its
+// own row free of bank conflicts.
+//
+// What bounds it: the chain of one value after the other (about 70 cycles in
+// fp32, 25 in fp64) against the warps the shared memory allows, and the length
+// of the runs in DRAM.  Measured on B200, 2^26 values, own differences, one
+// 16-value piece per block at a time (the kernel below) -> here: fp32 93.5 -> 72.8
+// us, fp64 153 -> 110.5 us; block 0's differences 67.3 -> 60.3 and 120 -> 101 us.
+// Runs of 32 bytes straight from registers took 115 / 171 us, of 128 bytes 75.8 /
+// 135 us, fp64 with 64 instead of 128 codes per stage 117 us, fp32 with 128
+// instead of 64 codes 82.5 us.
+//
+// For fp32 the sum is a double rounded to float at every step.  RND rounds it
+// by integer arithmetic on its bits (nearest, ties to even, at the 29 bits a
+// float drops) instead of two conversions in the chain from one value to the
+// next; it holds for sums that are zero or normal floats, which the caller
+// guarantees from the step's size.  Codes become doubles with one addition:
+// code + 2^15 sits in the low word of 2^52 + code + 2^15.
+template<class T, bool RND>
+struct legacy_sum
+{
+  double s = 0.0; // the running sum, exactly a T
+
+  // the T value (off the chain)
+  __device__ __forceinline__ T value() const
+  {
+    if constexpr (sizeof(T) == 4)
+      return __double2float_rn(s);
+    else
+      return s;
+  }
+  __device__ __forceinline__ void round_to_T()
+  {
+    if constexpr (sizeof(T) == 4) {
+      if constexpr (RND) {
+        const std::uint32_t lo = (std::uint32_t)__double2loint(s);
+        const std::uint32_t hi = (std::uint32_t)__double2hiint(s);
+        // half up, then an exact half whose kept part was even goes back down
+        const std::uint32_t keep = (lo & 0x3FFFFFFFu) == 0x10000000u ? 0xC0000000u : 0xE0000000u;
+        const std::uint64_t u = (((std::uint64_t)hi << 32) | lo) + 0x10000000u;
+        s = __hiloint2double((int)(u >> 32), (int)((std::uint32_t)u & keep));
+      } else {
+        s = (double)__double2float_rn(s);
+      }
+    }
+  }
+};
+
+// code as a double times ebx2, rounded as one product
+__device__ __forceinline__ double legacy_term(std::uint32_t code_plus_2p15, double ebx2)
+{
+  return __dmul_rn(__dadd_rn(__hiloint2double(0x43300000, (int)code_plus_2p15), -4503599627403264.0), ebx2);
+}
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* g)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((std::uint32_t)__cvta_generic_to_shared(smem)), "l"(g)
+               : "memory");
+}
+
+template<class T, bool OWN, bool RND>
+__global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t* __restrict__ in, std::uint64_t n,
+                                                             double ebx2, T* __restrict__ y)
+{
+  constexpr int VO = 64;                        // values per block and part
+  constexpr int CS = sizeof(T) == 4 ? 64 : 128; // codes per block and stage
+  constexpr int kOutBytes = VO * (int)sizeof(T);
+  constexpr int kRowBytes = kOutBytes + 16;         // a block's row of values
+  constexpr int CROW = 2 * CS + 16;                 // a block's row of codes
+  constexpr int PV = 16 / (int)sizeof(T);           // values per 16 bytes
+  constexpr int LPC = CS / 8, LPO = kOutBytes / 16; // threads per row of codes, of values
+  __shared__ __align__(16) std::uint8_t s_out[32 * kRowBytes];
+  __shared__ __align__(16) std::uint8_t s_in[OWN ? 2 * 32 * CROW : kLegacyBlock * 2];
+  const int lane = threadIdx.x;
+  const std::uint64_t v0 = (std::uint64_t)blockIdx.x * (32 * kLegacyBlock); // the CTA's first value
+  const int full = (int)min((std::uint64_t)32, (n - v0) / kLegacyBlock);    // its whole blocks
+  const std::uint64_t g0 = v0 + (std::uint64_t)lane * kLegacyBlock;         // this thread's block
+  if constexpr (!OWN) { // block 0's codes, which every block adds
+    for (int i = lane; i < kLegacyBlock; i += 32)
+      reinterpret_cast<std::int16_t*>(s_in)[i] = (std::uint64_t)i < n ? in[i] : (std::int16_t)0;
+    __syncwarp();
+  }
+  const std::int16_t* src = in + v0 + (lane / LPC) * kLegacyBlock + (lane % LPC) * 8;
+  std::uint8_t* s_src = s_in + (lane / LPC) * CROW + (lane % LPC) * 16;
+  auto issue = [&](int stage) {
+    if constexpr (OWN) {
+      if (stage < kLegacyBlock / CS) {
+#pragma unroll
+        for (int i = 0; i < LPC; ++i)
+          if ((32 / LPC) * i + lane / LPC < full)
+            cp_async16(s_src + (stage & 1) * (32 * CROW) + (32 / LPC) * i * CROW,
+                       src + stage * CS + (32 / LPC) * i * kLegacyBlock);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+  };
+  T* dst = y + v0 + (lane / LPO) * kLegacyBlock + (lane % LPO) * PV;
+  const std::uint8_t* s_dst = s_out + (lane / LPO) * kRowBytes + (lane % LPO) * 16;
+  legacy_sum<T, RND> acc;
+  issue(0);
+#pragma unroll 1
+  for (int part = 0; part < kLegacyBlock / VO; ++part) {
+    if constexpr (OWN) {
+      if (part * VO % CS == 0) {
+        issue(part * VO / CS + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+      }
+    }
+    const std::uint8_t* codes =
+      OWN ? s_in + (part * VO / CS & 1) * (32 * CROW) + lane * CROW + part * VO % CS * 2 : s_in + part * VO * 2;
+#pragma unroll
+    for (int h = 0; h < VO; h += 8) {
+      const uint4 c4 = *reinterpret_cast<const uint4*>(codes + h * 2);
+      std::uint32_t w[4] = { c4.x, c4.y, c4.z, c4.w };
+      if (!OWN && h == 0 && part == 0 && lane < full)
+        w[0] = (w[0] & 0xFFFF0000u) | (std::uint16_t)in[g0]; // the block's own first value
+#pragma unroll
+      for (int p = 0; p < 8; p += PV) {
+        std::uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < PV; ++k) {
+          const int i = p + k;
+          const std::uint32_t b = w[i / 2] ^ 0x80008000u; // codes + 2^15
+          const double t = legacy_term((i & 1) ? b >> 16 : b & 0xFFFFu, ebx2);
+          if (h == 0 && i == 0 && part == 0)
+            acc.s = t;
+          else
+            acc.s = __dadd_rn(t, acc.s);
+          acc.round_to_T();
+          if constexpr (sizeof(T) == 4) {
+            v[k] = __float_as_uint(acc.value());
+          } else {
+            v[2 * k] = (std::uint32_t)__double2loint(acc.s);
+            v[2 * k + 1] = (std::uint32_t)__double2hiint(acc.s);
+          }
+        }
+        *reinterpret_cast<uint4*>(s_out + lane * kRowBytes + (h + p) * (int)sizeof(T)) =
+          make_uint4(v[0], v[1], v[2], v[3]);
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < LPO; ++i)
+      if ((32 / LPO) * i + lane / LPO < full)
+        __stcs(reinterpret_cast<uint4*>(dst + part * VO + (32 / LPO) * i * kLegacyBlock),
+               *reinterpret_cast<const uint4*>(s_dst + (32 / LPO) * i * kRowBytes));
+    __syncwarp(); // the part has left; its codes' buffer is free
+  }
+  if (lane == full && g0 < n) { // the array's last, partial block
+    for (int i = 0; g0 + i < n; ++i) {
+      const std::int16_t q = OWN || i == 0 ? in[g0 + i] : reinterpret_cast<const std::int16_t*>(s_in)[OWN ? 0 : i];
+      const double t = __dmul_rn((double)q, ebx2);
+      acc.s = i == 0 ? t : __dadd_rn(t, acc.s);
+      acc.round_to_T();
+      y[g0 + i] = acc.value();
+    }
+  }
+}
+
+// Blocks for pointers off the 32-byte layout: 64 blocks per CTA, values through
+// shared memory 16 per block at a time and stored one by one, so the stores are
+// coalesced whatever the alignment.
 template<class T, bool OWN>
 __global__ void __launch_bounds__(kDecBlocks) k_frsz1_decompress(const std::int16_t* __restrict__ in, std::uint64_t n,
                                                                   double ebx2, T* __restrict__ y, bool vec)
@@ -315,6 +482,21 @@ int legacy_decompress(double eps, const void* d_in, std::uint64_t n, void* d_val
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, (nb + kDecBlocks - 1) / kDecBlocks);
   const auto* q = static_cast<const std::int16_t*>(d_in);
   T* y = static_cast<T*>(d_values);
+  if (reinterpret_cast<std::uintptr_t>(d_in) % 32 == 0 && reinterpret_cast<std::uintptr_t>(d_values) % 32 == 0) {
+    // RND: a nonzero sum of a product q * 2eps and a float is at least an ulp of
+    // the product, 2^-52 * 2eps, and at most 256 * 2^15 * 2eps: normal floats for
+    // 2eps in [2^-64, 2^96]
+    const double s2 = eps * 2;
+    const unsigned warps = (unsigned)std::max<std::uint64_t>(1, (nb + 31) / 32);
+    const bool rnd = sizeof(T) == 4 && s2 >= 0x1p-64 && s2 <= 0x1p96;
+    if (own)
+      rnd ? k_frsz1_decompress_vec<T, true, true><<<warps, 32, 0, s>>>(q, n, s2, y)
+          : k_frsz1_decompress_vec<T, true, false><<<warps, 32, 0, s>>>(q, n, s2, y);
+    else
+      rnd ? k_frsz1_decompress_vec<T, false, true><<<warps, 32, 0, s>>>(q, n, s2, y)
+          : k_frsz1_decompress_vec<T, false, false><<<warps, 32, 0, s>>>(q, n, s2, y);
+    return cuda_status(cudaGetLastError(), "legacy decompress launch");
+  }
   const bool vec = reinterpret_cast<std::uintptr_t>(d_in) % 16 == 0;
   if (own)
     k_frsz1_decompress<T, true><<<grid, kDecBlocks, 0, s>>>(q, n, eps * 2, y, vec);
