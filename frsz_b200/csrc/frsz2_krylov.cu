@@ -7,12 +7,11 @@
 //   frsz2_basis_dot:  h[j] = sum_i V_j[i] * w[i]           j < m
 //   frsz2_basis_axpy: y[i] = y[i] + sum_j c[j] * V_j[i]     (j in order 0..m-1)
 //
-// dot: CTA b owns a contiguous element range; it stages its slice of w in
-// shared memory once and streams every basis vector's slice through it (the
-// basis and w are each read once).  Per-warp partial sums per vector go to
-// shared memory; each CTA writes its m partials to the caller's workspace and
-// the last CTA to finish (a ticket counter in the workspace) adds them in CTA
-// order, so the result does not depend on scheduling.
+// dot: a warp takes a group of vectors over a slice of the positions, reads
+// each position of w once for the whole group, and writes one sum per vector;
+// a second kernel adds a vector's sums in slice order, so the result does not
+// depend on scheduling.  axpy: a thread holds its values of y in registers and
+// adds the vectors to them one after the other.
 #include "frsz2_fast.cuh"
 #include "frsz2_launch.hpp"
 
@@ -25,25 +24,9 @@ namespace frsz2b {
 namespace {
 
 constexpr int kMaxBasis = FRSZ2_MAX_BASIS;
-constexpr int kKT = 256;            // threads per CTA
-constexpr int kSub = 3072;          // w values staged per step (24 KiB)
-#ifndef FRSZ2_KRYLOV_JB
-#define FRSZ2_KRYLOV_JB 4
-#endif
-#ifndef FRSZ2_KRYLOV_MIN_CTAS
-#define FRSZ2_KRYLOV_MIN_CTAS 4
-#endif
-// Basis vectors whose loads are in flight together, per kernel and width.
-// Measured on B200 (100 vectors of 2^22 values, 4 CTAs per SM): the dot is
-// fastest with 4 at 32 bits (0.89 of HBM against 0.83 with 6) and with 6 at 16
-// and 24 bits (0.48 against 0.46, 0.68 against 0.66); the axpy with 6 at 16, 24
-// and 32 bits (0.66 against 0.61, 0.87 against 0.82, 1.03 against 1.02).  At
-// 21 bits 6 spills registers and halves the speed; 21, 48 and 64 bits keep
-// FRSZ2_KRYLOV_JB.
-constexpr int kJB = FRSZ2_KRYLOV_JB;
-__host__ __device__ constexpr int jb_dot(int bits) { return bits == 16 || bits == 24 ? 6 : kJB; }
-__host__ __device__ constexpr int jb_axpy(int bits) { return bits == 16 || bits == 24 || bits == 32 ? 6 : kJB; }
-constexpr int kMinCtas = FRSZ2_KRYLOV_MIN_CTAS; // resident CTAs per SM the register budget must allow
+constexpr int kKT = 256;              // threads per CTA
+constexpr int kKW = kKT / 32;         // warps per CTA
+constexpr int kSub = 3072;            // positions per partial sum that the workspace has room for
 
 struct BasisParams
 {
@@ -57,699 +40,412 @@ struct BasisGeo
   int log2E;
 };
 
-#ifndef FRSZ2_KRYLOV_NOCVT
-#define FRSZ2_KRYLOV_NOCVT 1
-#endif
-
-// Values of widths up to 32 bits without an integer-to-double conversion,
-// exactly the values fast_decode_loaded gives.  With t = code << (32 - BITS)
-// (sign at bit 31) and m = max(t << 1, 1), a value is m * 2^(be-31): for a
-// nonzero magnitude m = mag * 2^(33-BITS), so m * 2^(be-31) =
-// mag * 2^(be-BITS+2); for a zero magnitude m = 1 gives the decoder's
-// 2^(be-31).  m * 2^(be-31) = D - 2^(be+21) exactly, where D has exponent
-// be+21 and m in the low 32 bits of its mantissa (m < 2^32; the subtraction
-// of two doubles within a factor of 2 is exact).  Needs be+1044 to be a
-// normal exponent field and be in the plain range: be in [-959, 1002].
-// The value's sign goes onto the other factor of the product (sign_onto).
-template<int BITS>
-__device__ __forceinline__ bool nocvt_block(std::int64_t be)
+// Values per lane.  Eight share one exponent load, one range test and the
+// address arithmetic; above 32 bits eight values' codes take too many registers
+// for several vectors in flight.  Blocks of 4 values take four at every width.
+__host__ __device__ constexpr int basis_nv(int bits)
 {
-  return FRSZ2_KRYLOV_NOCVT && BITS <= 32 && be >= -959 && be <= 1002;
+  return bits <= 32 ? 8 : 4;
 }
 
-__device__ __forceinline__ double nocvt_magnitude(std::uint32_t t, int hi, double base)
+// Vectors whose loads a warp has in flight together, and the CTAs per SM that
+// the register budget must allow.  Swept on B200 over 1, 2, 4, 8 x 2..6 (dot, us
+// at 4 x 3 / 4 x 4 / 2 x 3 / 2 x 4): 100 vectors of 2^22 values at 32 bits 253 /
+// 326 (spills) / 316 / 256, at 16 bits 195 / 172 / 258 / 226; 50 of 2^21 at 21
+// bits 75.4 / 86.9 / 88.3 / 75.5, 24 bits 65.2 / 62.2 / 77.8 / 71.9, 48 bits 106 /
+// 105 / 113 / 112, 64 bits 213 / 312 / 161 / 195.  One or two vectors take a
+// variant of two: 1 vector of 2^22 at 32 bits 14.7 -> 12.0 us.
+__host__ __device__ constexpr int dot_jb(int bits) { return bits > 48 ? 2 : 4; }
+__host__ __device__ constexpr int dot_ctas(int bits, int nv, int jb)
 {
-  const std::uint32_t m = max(t << 1, 1u);
-  return __hiloint2double(hi, (int)m) - base;
+  if (bits > 48) return 3;
+  if (jb == 2 || nv == 4) return 4;
+  return bits == 21 || bits == 32 ? 3 : 4;
+}
+// axpy over 2..12 x 2..4 (us): 16 bits 6 x 3 170, 5 x 3 179, 3 x 4 182, 4 x 3 230;
+// 21 bits 5 x 3 67.1, 4 x 3 67.8; 24 bits 3 x 4 62.0, 4 x 3 65.3; 32 bits 4 x 3
+// 262, 3 x 4 265, 6 x 3 366 (spills); 48 bits 5 x 3 103, 4 x 3 118; 64 bits 5 x 3
+// 132, 4 x 3 133; four values per lane, 32 bits 6 x 4 45.7, 5 x 3 49.6.
+__host__ __device__ constexpr int axpy_jb(int bits, int nv)
+{
+  if (nv == 4 && bits <= 32) return 6;
+  return bits == 16 ? 6 : bits == 24 ? 3 : bits == 32 ? 4 : 5;
+}
+__host__ __device__ constexpr int axpy_ctas(int bits, int nv)
+{
+  return (nv == 4 && bits <= 32) || bits == 24 ? 4 : 3;
 }
 
-__device__ __forceinline__ double sign_onto(double x, std::uint32_t t)
+// One vector's codes of a lane's NV consecutive values, and their exponent.
+template<int BITS, int NV>
+struct basis_lane
 {
-  return __hiloint2double(__double2hiint(x) ^ (int)(t & 0x80000000u), __double2loint(x));
-}
+  static constexpr int SEG = NV * BITS; // bits
+  static constexpr int NW = (SEG + 31) / 32;
+  static constexpr bool ALIGNED = SEG % 32 == 0;
+  using exp_t = std::conditional_t<(BITS > 32), std::int64_t, std::int32_t>;
+  std::uint32_t w[ALIGNED ? NW : NW + 1];
+  exp_t be;
+};
 
-// acc + sum over the lane's values of v[k] * wv[k], FMAs in value order.
-template<int BITS>
-__device__ __forceinline__ double lane_dot(const lane_words<double, BITS>& lw,
-                                           const double (&wv)[fast_cfg<double, BITS>::P], double acc)
+// NW words at p, aligned to 4 bytes or, with WIDE, to the largest power of two
+// dividing their bytes.  One load of 16 or 32 bytes takes them past the L1 cache
+// (each sector is read once, and w stays there); several go through it, since a
+// sector then serves more than one of them (21 bits, six loads: 97 -> 75 us), and
+// so do 8-byte ones (axpy of 30 vectors of 300,007 values, 16 bits: 7.5 -> 6.8 us).
+template<int NW, bool WIDE>
+__device__ __forceinline__ void ldg_words(const std::uint32_t* p, std::uint32_t* w)
 {
-  constexpr int P = fast_cfg<double, BITS>::P;
-  if constexpr (BITS <= 32) {
-    const std::int64_t be = lw.be;
-    if (nocvt_block<BITS>(be)) {
-      std::uint32_t c[P];
-      fast_codes_loaded<double, BITS>(lw, c);
-      const int hi = (int)((std::uint32_t)(be + 1044) << 20);
-      const double base = __hiloint2double(hi, 0);
+  constexpr int V = !WIDE ? 1 : NW % 8 == 0 ? 8 : NW % 4 == 0 ? 4 : NW % 2 == 0 ? 2 : 1;
+  if constexpr (V == NW && V >= 4) {
+    if constexpr (V == 8)
+      asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                   : "l"(p));
+    else
+      asm volatile("ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];"
+                   : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3])
+                   : "l"(p));
+  } else {
 #pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const std::uint32_t t = c[k] << (32 - BITS);
-        acc = fma(nocvt_magnitude(t, hi, base), sign_onto(wv[k], t), acc);
+    for (int i = 0; i < NW; i += V) {
+      if constexpr (V == 4) {
+        const uint4 t = __ldg(reinterpret_cast<const uint4*>(p + i));
+        w[i] = t.x;
+        w[i + 1] = t.y;
+        w[i + 2] = t.z;
+        w[i + 3] = t.w;
+      } else if constexpr (V == 2) {
+        const uint2 t = __ldg(reinterpret_cast<const uint2*>(p + i));
+        w[i] = t.x;
+        w[i + 1] = t.y;
+      } else {
+        w[i] = __ldg(p + i);
       }
-      return acc;
     }
   }
-  double v[P];
-  fast_decode_loaded<double, BITS>(lw, v);
+}
+
+// The codes at stream bit S of a vector (words at `words`) and the exponent at
+// `exp`; S is a multiple of NV * BITS.
+template<int BITS, int NV>
+__device__ __forceinline__ void basis_load(const std::uint8_t* exp, const std::uint8_t* words, std::uint64_t S,
+                                           basis_lane<BITS, NV>& l)
+{
+  using L = basis_lane<BITS, NV>;
+  constexpr int W = fast_cfg<double, BITS>::W;
+  l.be = (typename L::exp_t)load_exp(exp, W);
+  const std::uint32_t* p = reinterpret_cast<const std::uint32_t*>(words) + (S >> 5);
+  ldg_words<L::NW, L::ALIGNED>(p, l.w);
+  if constexpr (!L::ALIGNED) l.w[L::NW] = ((int)(S & 31u) + L::SEG > 32 * L::NW) ? __ldg(p + L::NW) : 0u;
+}
+
+template<int K, int BITS, int N, int NV, class C>
+__device__ __forceinline__ void basis_codes(const std::uint32_t (&seg)[N], C (&c)[NV])
+{
+  if constexpr (K < NV) {
+    c[K] = (C)get_bits<K * BITS, BITS>(seg);
+    basis_codes<K + 1, BITS>(seg, c);
+  }
+}
+
+// Values of widths up to 48 bits without an integer-to-double conversion,
+// exactly the values of the decoder.  D - base, both doubles of exponent field
+// F = be + 1044 (or be + 1029), where D has the magnitude in the low bits of its
+// mantissa, so the subtraction is exact.
+//   up to 32 bits: with t = code << (32 - BITS) (sign at bit 31) the low word is
+//     max(t << 1, 1): a nonzero magnitude is mag * 2^(33-BITS), worth
+//     mag * 2^(be-BITS+2) at F = be + 1044; a zero magnitude gives the decoder's
+//     2^(be-31).
+//   33 to 48 bits: the magnitude shifted up to 47 bits, or 2^15 when it is zero,
+//     at F = be + 1029 (a unit is 2^(be-46)).
+// Needs F to be a normal exponent field and be in the plain range:
+// be in [-959, 1002].
+template<int BITS>
+__device__ __forceinline__ bool direct_exponent(std::int64_t be)
+{
+  return be >= -959 && be <= 1002;
+}
+
+template<int BITS, int NV>
+__device__ __forceinline__ void basis_values_direct(const basis_lane<BITS, NV>& l, int o, double (&v)[NV])
+{
+  using L = basis_lane<BITS, NV>;
+  using C = std::conditional_t<(BITS <= 32), std::uint32_t, std::uint64_t>;
+  std::uint32_t seg[L::NW + 1];
 #pragma unroll
-  for (int k = 0; k < P; ++k) acc = fma(v[k], wv[k], acc);
+  for (int i = 0; i < L::NW; ++i) {
+    if constexpr (L::ALIGNED)
+      seg[i] = l.w[i];
+    else
+      seg[i] = __funnelshift_r(l.w[i], l.w[i + 1], o);
+  }
+  seg[L::NW] = 0;
+  C c[NV];
+  basis_codes<0, BITS>(seg, c);
+  if constexpr (BITS <= 32) {
+    const int hi = (int)((std::uint32_t)(l.be + 1044) << 20);
+    const double base = __hiloint2double(hi, 0);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const std::uint32_t t = c[k] << (32 - BITS);
+      const double d = __hiloint2double(hi, (int)max(t << 1, 1u)) - base;
+      v[k] = __hiloint2double(__double2hiint(d) ^ (int)(t & 0x80000000u), __double2loint(d));
+    }
+  } else {
+    static_assert(BITS <= 48, "magnitudes below 2^47");
+    const std::uint32_t hi = (std::uint32_t)(l.be + 1029) << 20;
+    const double base = __hiloint2double((int)hi, 0);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const std::uint64_t t = c[k] << (48 - BITS); // sign at bit 47
+      std::uint32_t lo = (std::uint32_t)t;
+      const std::uint32_t up = (std::uint32_t)(t >> 32) & 0x7FFFu;
+      if ((lo | up) == 0) lo = 0x8000u;
+      const double d = __hiloint2double((int)(hi | up), (int)lo) - base;
+      v[k] = __hiloint2double(__double2hiint(d) ^ (int)((std::uint32_t)(t >> 16) & 0x80000000u), __double2loint(d));
+    }
+  }
+}
+
+// The same through the decoder's own arithmetic, for every exponent.
+template<int BITS, int NV>
+__device__ __forceinline__ void basis_values_any(const basis_lane<BITS, NV>& l, int o, double (&v)[NV])
+{
+  using L = basis_lane<BITS, NV>;
+  using C = typename fast_cfg<double, BITS>::C;
+  std::uint32_t seg[L::NW + 1];
+#pragma unroll
+  for (int i = 0; i < L::NW; ++i) {
+    if constexpr (L::ALIGNED)
+      seg[i] = l.w[i];
+    else
+      seg[i] = __funnelshift_r(l.w[i], l.w[i + 1], o);
+  }
+  seg[L::NW] = 0;
+  C c[NV];
+  basis_codes<0, BITS>(seg, c);
+  const std::int64_t be = l.be;
+  if (plain_exponent<double>(be)) {
+    const double inv = pow2<double>((int)be - BITS + 2);
+    const std::uint64_t zero_bits = (std::uint64_t)(be + 992) << 52;
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = from_bits<double>(decode_plain<double, BITS>(c[k], inv, zero_bits));
+  } else {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) v[k] = from_code<double>((std::uint64_t)c[k], be, BITS);
+  }
+}
+
+constexpr bool has_direct(int bits) { return bits <= 48; }
+
+// acc + sum of v[k] * w[k], k < cnt, in order: a lane of a step that holds an
+// exponent outside the direct range (loads again, off the fast path).  JB gives
+// each kernel its own copy: nvcc 12.9 fails on one that is shared by kernels of
+// different register bounds.
+template<int BITS, int NV, int JB>
+__device__ __noinline__ double slow_lane_dot(const std::uint8_t* exp, const std::uint8_t* words, std::uint64_t S,
+                                             const double* w, int cnt, double acc)
+{
+  basis_lane<BITS, NV> l;
+  basis_load<BITS, NV>(exp, words, S, l);
+  double v[NV];
+  basis_values_any<BITS, NV>(l, (int)(S & 31u), v);
+#pragma unroll
+  for (int k = 0; k < NV; ++k)
+    if (k < cnt) acc = fma(v[k], __ldg(w + k), acc);
   return acc;
 }
 
-// acc[k] + cj * v[k] for the lane's values.
-template<int BITS>
-__device__ __forceinline__ void lane_axpy(const lane_words<double, BITS>& lw, double cj,
-                                          double (&acc)[fast_cfg<double, BITS>::P])
+// y[k] + c * v[k] on a lane's values of y in memory, k < cnt.
+template<int BITS, int NV>
+__device__ __noinline__ void slow_lane_axpy(const std::uint8_t* exp, const std::uint8_t* words, std::uint64_t S,
+                                            double c, double* y)
 {
-  constexpr int P = fast_cfg<double, BITS>::P;
-  if constexpr (BITS <= 32) {
-    const std::int64_t be = lw.be;
-    if (nocvt_block<BITS>(be)) {
-      std::uint32_t c[P];
-      fast_codes_loaded<double, BITS>(lw, c);
-      const int hi = (int)((std::uint32_t)(be + 1044) << 20);
-      const double base = __hiloint2double(hi, 0);
+  basis_lane<BITS, NV> l;
+  basis_load<BITS, NV>(exp, words, S, l);
+  double v[NV];
+  basis_values_any<BITS, NV>(l, (int)(S & 31u), v);
 #pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const std::uint32_t t = c[k] << (32 - BITS);
-        acc[k] = fma(sign_onto(cj, t), nocvt_magnitude(t, hi, base), acc[k]);
-      }
-      return;
-    }
-  }
-  double v[P];
-  fast_decode_loaded<double, BITS>(lw, v);
-#pragma unroll
-  for (int k = 0; k < P; ++k) acc[k] = fma(cj, v[k], acc[k]);
+  for (int k = 0; k < NV; ++k) y[k] = fma(c, v[k], y[k]);
 }
 
-template<int BITS>
-__global__ void __launch_bounds__(kKT, kMinCtas)
-  k_basis_dot(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ w,
-              std::uint64_t chunk, double* __restrict__ partials, unsigned int* __restrict__ ticket,
-              double* __restrict__ h)
+// Sums of N (a power of two up to 32) values over the warp in a fixed order:
+// each exchange halves the values a lane carries, so N values cost N - 1 +
+// log2(32 / N) exchanges instead of 5 N.  Returns the sum of value
+// (lane * N) / 32.
+template<int N>
+__device__ __forceinline__ double warp_sums(double (&a)[N])
 {
-  constexpr int P = fast_cfg<double, BITS>::P;
-  constexpr int JB = jb_dot(BITS);
-  __shared__ double s_w[kSub];
-  __shared__ double s_acc[kKT / 32][kMaxBasis];
-  __shared__ bool s_last;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int j = lane; j < m; j += 32) s_acc[warp][j] = 0.0;
-
-  const std::uint64_t c0 = (std::uint64_t)blockIdx.x * chunk;
-  const std::uint64_t c1 = c0 + chunk < g.n ? c0 + chunk : g.n;
-  for (std::uint64_t s0 = c0; s0 < c1; s0 += kSub) {
-    const int len = (int)((c1 - s0) < (std::uint64_t)kSub ? (c1 - s0) : (std::uint64_t)kSub);
-    __syncthreads(); // previous slice fully consumed
-    for (int i = tid; i < len; i += kKT) s_w[i] = __ldg(w + s0 + i);
-    __syncthreads();
-    // JB vectors at a time: all their loads are issued before any decode
-    for (int j0 = 0; j0 < m; j0 += JB) {
-      double acc[JB];
-#pragma unroll
-      for (int jj = 0; jj < JB; ++jj) acc[jj] = 0.0;
-      for (int i = tid * P; i < len; i += kKT * P) {
-        lane_words<double, BITS> lw[JB];
-#pragma unroll
-        for (int jj = 0; jj < JB; ++jj)
-          if (j0 + jj < m) {
-            const std::uint8_t* buf = bp.buf[j0 + jj];
-            fast_load_lane<double, BITS>(buf, buf + g.exp_bytes, g.log2E, s0 + (std::uint64_t)i, lw[jj]);
-          }
-        double wv[P];
-#pragma unroll
-        for (int k = 0; k < P; ++k) wv[k] = i + k < len ? s_w[i + k] : 0.0;
-#pragma unroll
-        for (int jj = 0; jj < JB; ++jj)
-          if (j0 + jj < m) acc[jj] = lane_dot<BITS>(lw[jj], wv, acc[jj]);
-      }
-#pragma unroll
-      for (int jj = 0; jj < JB; ++jj) {
-        double a = acc[jj];
-#pragma unroll
-        for (int s = 16; s > 0; s >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, s);
-        if (lane == 0 && j0 + jj < m) s_acc[warp][j0 + jj] += a;
-      }
-    }
-  }
-  __syncthreads();
-  for (int j = tid; j < m; j += kKT) {
-    double p = 0.0;
-#pragma unroll
-    for (int q = 0; q < kKT / 32; ++q) p += s_acc[q][j];
-    partials[(std::uint64_t)blockIdx.x * m + j] = p;
-  }
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (s_last) {
-    __threadfence();
-    for (int j = tid; j < m; j += kKT) {
-      double sum = 0.0;
-      for (unsigned b = 0; b < gridDim.x; ++b) sum += __ldcg(partials + (std::uint64_t)b * m + j);
-      h[j] = sum;
-    }
-    if (tid == 0) *ticket = 0u; // ready for the next call
-  }
-}
-
-// Place of value i of a slice of w in shared memory: 16-byte chunk q = i / 2
-// at q ^ ((q >> 3) & 1).
-__device__ __forceinline__ int dot_swz(int i) { return (((i >> 1) ^ ((i >> 4) & 1)) << 1) | (i & 1); }
-
-// Dot with work handed out at run time: an item is a group of vg vectors over
-// a slice of kSub values; CTAs take items from a counter in the workspace, so
-// SMs that run slower take fewer (a fixed split measured a 10 % spread of SM
-// busy time), and write each (vector, slice) sum to its own place in
-// partials; k_basis_dot_final adds them in slice order, so h does not depend
-// on which CTA took which item, on the grid or on vg.
-template<int BITS>
-__global__ void __launch_bounds__(kKT, kMinCtas)
-  k_basis_dot_dyn(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ w,
-                  unsigned int ns, int vg, double* __restrict__ partials, unsigned int* __restrict__ next_item)
-{
-  constexpr int P = fast_cfg<double, BITS>::P;
-  constexpr int JB = jb_dot(BITS);
-  __shared__ double s_w[kSub];
-  __shared__ double s_acc[kKT / 32][kMaxBasis];
-  __shared__ unsigned int s_item;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned int groups = (unsigned)((m + vg - 1) / vg);
-  const unsigned int items = ns * groups;
-
-  for (;;) {
-    if (tid == 0) s_item = atomicAdd(next_item, 1u);
-    __syncthreads(); // also: the previous item's s_w / s_acc are consumed
-    const unsigned int it = s_item;
-    if (it >= items) break;
-    // an item: vectors [jb, je) over slice sl
-    const unsigned int sl = it / groups;
-    const int jb = (int)(it - sl * groups) * vg, je = min(jb + vg, m);
-    const std::uint64_t s0 = (std::uint64_t)sl * kSub;
-    const int len = (int)((g.n - s0) < (std::uint64_t)kSub ? (g.n - s0) : (std::uint64_t)kSub);
-    // 16-byte chunks of w swizzled (chunk q at q ^ ((q >> 3) & 1)), so the
-    // 32-byte runs of a warp's lanes fall on distinct banks
-    for (int i = tid; i < len; i += kKT) s_w[dot_swz(i)] = __ldg(w + s0 + i);
-    __syncthreads();
-    // JB vectors at a time: all their loads are issued before any decode
-    for (int j0 = jb; j0 < je; j0 += JB) {
-      double acc[JB];
-#pragma unroll
-      for (int jj = 0; jj < JB; ++jj) acc[jj] = 0.0;
-      for (int i = tid * P; i < len; i += kKT * P) {
-        lane_words<double, BITS> lw[JB];
-#pragma unroll
-        for (int jj = 0; jj < JB; ++jj)
-          if (j0 + jj < je) {
-            const std::uint8_t* buf = bp.buf[j0 + jj];
-            fast_load_lane<double, BITS>(buf, buf + g.exp_bytes, g.log2E, s0 + (std::uint64_t)i, lw[jj]);
-          }
-        double wv[P];
-        if (i + P <= len) {
-          const double2* wr = reinterpret_cast<const double2*>(s_w) + (i >> 1);
-          const int f = (lane >> 2) & 1; // i >> 1 = 2 * tid + 512 * pass: chunk swizzle (tid >> 2) & 1
-          const double2 wa = wr[f], wb = wr[1 - f];
-          wv[0] = wa.x;
-          wv[1] = wa.y;
-          wv[2] = wb.x;
-          wv[3] = wb.y;
-        } else {
-#pragma unroll
-          for (int k = 0; k < P; ++k) wv[k] = i + k < len ? s_w[dot_swz(i + k)] : 0.0;
-        }
-#pragma unroll
-        for (int jj = 0; jj < JB; ++jj)
-          if (j0 + jj < je) acc[jj] = lane_dot<BITS>(lw[jj], wv, acc[jj]);
-      }
-#pragma unroll
-      for (int jj = 0; jj < JB; ++jj) {
-        double a = acc[jj];
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, sh);
-        if (lane == 0 && j0 + jj < je) s_acc[warp][j0 + jj] = a; // each (warp, vector) once per item
-      }
-    }
-    __syncthreads();
-    // this item's sums, vector-major: partials[j * ns + sl]
-    for (int j = jb + tid; j < je; j += kKT) {
-      double p = 0.0;
-#pragma unroll
-      for (int q = 0; q < kKT / 32; ++q) p += s_acc[q][j];
-      partials[(std::uint64_t)j * ns + sl] = p;
-    }
-  }
-}
-
-// h[j] = sum over slices of partials[j * ns + slice], in a fixed order; one
-// CTA per vector.  Leaves the slice counter at zero for the next call.
-__global__ void __launch_bounds__(kKT)
-  k_basis_dot_final(const double* __restrict__ partials, unsigned int ns, double* __restrict__ h,
-                    unsigned int* __restrict__ next_slice)
-{
-  __shared__ double s_red[kKT / 32];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const double* pj = partials + (std::uint64_t)blockIdx.x * ns;
-  double sum = 0.0;
-  for (unsigned int b = tid; b < ns; b += kKT) sum += __ldcg(pj + b);
-#pragma unroll
-  for (int sh = 16; sh > 0; sh >>= 1) sum += __shfl_down_sync(0xFFFFFFFFu, sum, sh);
-  if (lane == 0) s_red[warp] = sum;
-  __syncthreads();
-  if (tid == 0) {
-    double t = 0.0;
-#pragma unroll
-    for (int q = 0; q < kKT / 32; ++q) t += s_red[q];
-    h[blockIdx.x] = t;
-    if (blockIdx.x == 0) *next_slice = 0u;
-  }
-}
-
-// ---------------------------------------------------------------- dot over per-warp copy rings
-//
-// The register kernel above keeps each thread's next codes in registers, so
-// the loads a warp has in flight are bounded by its register budget, and it
-// waits on them (long scoreboard) for most of its time.  Here each warp
-// streams its codes and exponents through its own ring of kRD shared-memory
-// slots with bulk asynchronous copies (cp.async.bulk, completion counted on one
-// mbarrier per slot): lane 0 issues a stage's copies kRD stages ahead of the
-// warp's decode, so a stage's latency is covered by the stages before it and
-// no register is held for a load in flight.
-//
-// Work is the same (slice, vector group) items as above, taken from a counter;
-// the CTA claims each item two ahead, so a warp's ring runs on into the next
-// item's stages while the CTA adds up the current one and stages the next
-// slice of w.  Inside an item, a unit is a pair of vectors over a range of the
-// slice's warp rows; warp k takes units k, k + 8, ... .  A stage is R warp rows
-// (128 values each) of both vectors of a unit: their codes and the 16-byte
-// aligned span of exponents that covers them.  Each unit's lane-summed result
-// goes to its own place, and the item's sum per vector adds them in a fixed
-// order, so h does not depend on scheduling.  w's slice sits in shared memory
-// with its 16-byte chunks swizzled (chunk q at q ^ ((q >> 3) & 1)), so the
-// 32-byte runs the lanes of a warp read fall on distinct banks.
-//
-// Every mbarrier wait is bounded (2 s): a wait that runs out sets an error
-// flag in the workspace, the CTA stops at its next item boundary, and the
-// dot then returns NaN for every h[j].
-
-constexpr int kRW = 8;                 // warps per CTA
-constexpr int kRT = kRW * 32;          // threads per CTA
-constexpr int kRSlice = kSub;          // values per item (24 warp rows)
-constexpr int kRRow = 128;             // values per warp row: 32 lanes x 4
-constexpr int kRMaxGroup = 32;         // vectors per item at most
-// Stages per warp ring.  Measured on B200 (100 vectors of 2^22 values, 64
-// bits): the time does not change with 2, 3 or 4 stages of the same size and
-// drops by a fifth when a stage doubles (1 -> 2 warp rows per vector); the
-// shared memory of two stages of 2 rows keeps 2 CTAs per SM.
-constexpr int kRD = 2;
-constexpr int kRPart = 2 * kRMaxGroup; // unit sums per item, then the partial-row sums
-
-template<int BITS>
-struct ring_shape
-{
-  static constexpr int RB = 16 * BITS; // code bytes of one warp row (a multiple of 16)
-  // warp rows per stage: two vectors' codes of a stage come to about 4 KiB
-  static constexpr int R = BITS <= 16 ? 8 : BITS <= 24 ? 6 : BITS <= 32 ? 4 : 2;
-  static constexpr int CODE = R * RB;  // code bytes per vector and stage
-  static constexpr int W = fast_cfg<double, BITS>::W;
-  static constexpr int Wb = W / 8;
-};
-
-// Bytes of one vector's exponent span in a slot: the 16-byte aligned span of
-// exponents covering R warp rows that start at any row.
-__host__ __device__ constexpr int ring_expw(int R, int log2E, int Wb)
-{
-  return ((((R * kRRow - 1) >> log2E) + 2) * Wb + 30 + 15) / 16 * 16;
-}
-
-__device__ __forceinline__ std::uint32_t smem_addr(const void* p)
-{
-  return (std::uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(std::uint64_t* bar, unsigned count)
-{
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive_expect_tx(std::uint64_t* bar, unsigned bytes)
-{
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ bool mbar_try_wait(std::uint64_t* bar, unsigned parity)
-{
-  unsigned done;
-  asm volatile("{\n\t.reg .pred p;\n\t"
-               "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-               "selp.u32 %0, 1, 0, p;\n\t}"
-               : "=r"(done)
-               : "r"(smem_addr(bar)), "r"(parity)
-               : "memory");
-  return done != 0;
-}
-
-// Global -> shared bulk copy (no multicast), completion counted on `bar`.
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, std::uint64_t* bar)
-{
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                 smem_addr(dst)),
-               "l"(src), "r"(bytes), "r"(smem_addr(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ std::uint64_t global_ns()
-{
-  std::uint64_t t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-// Waits for a slot's phase, at most `limit_ns`; every lane of the warp gets
-// the same answer.
-__device__ __forceinline__ bool ring_wait(std::uint64_t* bar, unsigned parity, std::uint64_t limit_ns)
-{
-  bool done = mbar_try_wait(bar, parity);
-  if (!done) {
-    const std::uint64_t t0 = global_ns();
-    while (!(done = mbar_try_wait(bar, parity)))
-      if (global_ns() - t0 > limit_ns) break;
-  }
-  return __all_sync(0xFFFFFFFFu, done);
-}
-
-struct RingItem
-{
-  std::uint64_t s0; // first value of the slice
-  int jb, G;        // vectors [jb, jb + G)
-  int P, C, RC;     // vector pairs, row chunks per pair, warp rows per chunk
-  int rows, len;    // whole warp rows in the slice, values in the slice
-};
-
-__device__ __forceinline__ RingItem ring_item(unsigned it, unsigned groups, int vg, int m, std::uint64_t n)
-{
-  RingItem r;
-  const unsigned sl = it / groups;
-  r.jb = (int)(it - sl * groups) * vg;
-  r.G = min(vg, m - r.jb);
-  r.s0 = (std::uint64_t)sl * kRSlice;
-  const std::uint64_t rem = n - r.s0;
-  r.len = rem < (std::uint64_t)kRSlice ? (int)rem : kRSlice;
-  r.rows = r.len / kRRow;
-  r.P = (r.G + 1) / 2;
-  r.C = r.P >= kRW ? 1 : (kRW + r.P - 1) / r.P; // at least one unit per warp
-  r.RC = (r.rows + r.C - 1) / r.C;
-  return r;
-}
-
-// One lane's codes of a warp row held in shared memory.
-template<int BITS>
-__device__ __forceinline__ void ring_lane_words(const std::uint8_t* row, int lane, lane_words<double, BITS>& lw)
-{
-  using Cfg = fast_cfg<double, BITS>;
-  constexpr int NW = Cfg::NW;
-  if constexpr (Cfg::ALIGNED) {
-    constexpr int LB = BITS / 2; // a lane's 4 codes in bytes
-    const std::uint8_t* p = row + lane * LB;
-    if constexpr (LB % 16 == 0) {
-#pragma unroll
-      for (int i = 0; i < NW / 4; ++i) {
-        const uint4 v = reinterpret_cast<const uint4*>(p)[i];
-        lw.w[4 * i] = v.x;
-        lw.w[4 * i + 1] = v.y;
-        lw.w[4 * i + 2] = v.z;
-        lw.w[4 * i + 3] = v.w;
-      }
-    } else if constexpr (LB % 8 == 0) {
-#pragma unroll
-      for (int i = 0; i < NW / 2; ++i) {
-        const uint2 v = reinterpret_cast<const uint2*>(p)[i];
-        lw.w[2 * i] = v.x;
-        lw.w[2 * i + 1] = v.y;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < NW; ++i) lw.w[i] = reinterpret_cast<const std::uint32_t*>(p)[i];
-    }
-    lw.o = 0;
+  const int lane = threadIdx.x & 31;
+  if constexpr (N == 1) {
+    return a[0];
   } else {
-    const int S = lane * 4 * BITS;
-    const std::uint32_t* q = reinterpret_cast<const std::uint32_t*>(row) + (S >> 5);
-    lw.o = S & 31;
+    constexpr int H = N / 2;
+    double b[H];
 #pragma unroll
-    for (int i = 0; i < NW; ++i) lw.w[i] = q[i];
-    lw.w[NW] = (lw.o + 4 * BITS > 32 * NW) ? q[NW] : 0u;
+    for (int i = 0; i < H; ++i) {
+      // the distance between the two halves of the lanes at this level
+      const bool up = (lane & 16) != 0;
+      const double send = up ? a[i] : a[i + H];
+      b[i] = (up ? a[i + H] : a[i]) + __shfl_xor_sync(0xFFFFFFFFu, send, 16);
+    }
+    if constexpr (H == 1) {
+      return b[0];
+    } else {
+      constexpr int Q = H / 2;
+      double c[Q];
+#pragma unroll
+      for (int i = 0; i < Q; ++i) {
+        const bool up = (lane & 8) != 0;
+        const double send = up ? b[i] : b[i + Q];
+        c[i] = (up ? b[i + Q] : b[i]) + __shfl_xor_sync(0xFFFFFFFFu, send, 8);
+      }
+      if constexpr (Q == 1) {
+        return c[0];
+      } else {
+        static_assert(Q == 2, "at most eight values");
+        const bool up = (lane & 4) != 0;
+        const double send = up ? c[0] : c[1];
+        return (up ? c[1] : c[0]) + __shfl_xor_sync(0xFFFFFFFFu, send, 4);
+      }
+    }
   }
 }
 
-template<int BITS>
-__global__ void __launch_bounds__(kRT, 2)
-  k_basis_dot_ring(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ w,
-                   unsigned int ns, int vg, int expw, int slot_bytes, double* __restrict__ partials,
-                   unsigned int* __restrict__ ctl)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Partial sums of the dot.  Unit u = slice * groups + group is JB vectors over
+// S positions, done by 2^lq warps of a CTA that take a part of the slice each;
+// a CTA's units are neighbouring groups of one slice, so its warps read w from
+// the L1 cache after the first.
+//
+// Bound by DRAM at 32 bits (253 us for 100 vectors of 2^22, 1.06 of the copy
+// bandwidth) and by instructions at 16 (10.8 per value, 172 us, 0.80; 280 us
+// and 18.1 before: four values per lane, w in shared memory behind two barriers
+// per slice, a warp-wide sum per vector every 12 values of a lane).
+template<int BITS, int NV, int JB>
+__global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
+  k_basis_dot(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ w, unsigned ns,
+              unsigned groups, unsigned S, int lq, double* __restrict__ partials)
 {
-  using S = ring_shape<BITS>;
-  constexpr int R = S::R, RB = S::RB, CODE = S::CODE, Wb = S::Wb;
-  extern __shared__ __align__(128) std::uint8_t smem[];
-  double* s_w = reinterpret_cast<double*>(smem);              // kRSlice values, chunk-swizzled
-  double* s_part = s_w + kRSlice;                             // kRPart
-  std::uint64_t* s_bar = reinterpret_cast<std::uint64_t*>(s_part + kRPart);
-  unsigned int* s_item = reinterpret_cast<unsigned int*>(s_bar + kRW * kRD); // 3 items, abort flag
-  std::uint8_t* s_ring = smem + ((kRSlice + kRPart) * 8 + kRW * kRD * 8 + 16 + 127) / 128 * 128;
-
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const unsigned int groups = (unsigned)((m + vg - 1) / vg);
-  const unsigned int items = ns * groups;
-  std::uint8_t* ring = s_ring + (std::size_t)warp * kRD * slot_bytes;
-  std::uint64_t* bar = s_bar + warp * kRD;
-  constexpr std::uint64_t kLimitNs = 2000000000ull;
-
-  if (lane == 0)
-    for (int s = 0; s < kRD; ++s) mbar_init(&bar[s], 1);
-  if (tid == 0) {
-    s_item[0] = atomicAdd(&ctl[0], 1u);
-    s_item[1] = atomicAdd(&ctl[0], 1u);
-    s_item[3] = 0u;
-  }
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  __syncthreads();
-
-  // w's slice of an item into s_w (zeros past the array), 16-byte chunks swizzled
-  auto stage_w = [&](unsigned it) {
-    const RingItem r = ring_item(it, groups, vg, m, g.n);
-    double2* sw2 = reinterpret_cast<double2*>(s_w);
-    for (int q = tid; q < kRSlice / 2; q += kRT) {
-      const int i = 2 * q;
-      const double a = i < r.len ? __ldg(w + r.s0 + i) : 0.0;
-      const double b = i + 1 < r.len ? __ldg(w + r.s0 + i + 1) : 0.0;
-      sw2[q ^ ((q >> 3) & 1)] = make_double2(a, b);
-    }
-  };
-  if (s_item[0] < items) stage_w(s_item[0]);
-
-  // ---- producer: the next stage of this warp's stream, kRD stages ahead.
-  // Per unit it keeps the two vectors' buffers and the next stage's first
-  // value; a stage then costs a few additions and lane 0's copies.
-  unsigned int issued = 0, consumed = 0;
-  int pk = 0;                           // item sequence number of the producer
-  RingItem pi = ring_item(s_item[0], groups, vg, m, g.n);
-  bool p_live = s_item[0] < items;      // the producer's item is a valid one
-  int pu = warp;                        // unit
-  int p_rows = 0;                       // warp rows of the unit not yet issued
-  std::uint64_t p_pos = 0;              // first value of the next stage
-  const std::uint8_t* p_buf0 = nullptr; // the unit's vectors
-  const std::uint8_t* p_buf1 = nullptr;
-  int p_nv = 0;
-  int ck = 0;                           // item sequence number of the consumer
-  bool ok = true;                       // no wait of this warp ran out
-  unsigned int drain_from = 0;          // the first stage not known to have landed, after a wait ran out
-  const int emask = (1 << g.log2E) - 1;
-
-  auto p_unit = [&]() {
-    if (pu >= pi.P * pi.C) {
-      p_rows = 0;
-      return;
-    }
-    const int c = pu % pi.C, pair = pu / pi.C;
-    const int r0 = c * pi.RC;
-    p_rows = max(0, min(pi.rows, r0 + pi.RC) - r0);
-    p_pos = pi.s0 + (std::uint64_t)r0 * kRRow;
-    const int j0 = pi.jb + 2 * pair;
-    p_nv = min(2, pi.G - 2 * pair);
-    p_buf0 = bp.buf[j0];
-    p_buf1 = bp.buf[p_nv > 1 ? j0 + 1 : j0];
-  };
-  if (p_live) p_unit();
-
-  // A stage to issue, moving over units and items; false when none is
-  // allowed yet (item ck + 2 is announced at the end of item ck) or none is left.
-  auto p_seek = [&]() -> bool {
-    while (p_live) {
-      if (p_rows > 0) return true;
-      if (pu + kRW < pi.P * pi.C) {
-        pu += kRW;
-        p_unit();
-        continue;
-      }
-      if (pk > ck) return false;
-      ++pk;
-      const unsigned int id = s_item[pk % 3];
-      p_live = id < items;
-      if (p_live) {
-        pi = ring_item(id, groups, vg, m, g.n);
-        pu = warp;
-        p_unit();
-      }
-    }
-    return false;
-  };
-  auto p_issue = [&]() {
-    const int slot = (int)(issued % kRD);
-    const int nr = min(R, p_rows);
-    if (lane == 0) {
-      const unsigned int cbytes = (unsigned)(nr * RB);
-      const std::uint64_t e0 = (p_pos >> g.log2E) * Wb;
-      const std::uint64_t e1 = (((p_pos + (std::uint64_t)nr * kRRow - 1) >> g.log2E) + 1) * Wb;
-      const std::uint64_t ws = e0 & ~15ull;
-      const unsigned int ebytes = (unsigned)(((e1 + 15) & ~15ull) - ws);
-      std::uint8_t* sp = ring + (std::size_t)slot * slot_bytes;
-      const std::uint64_t coff = g.exp_bytes + p_pos * (std::uint64_t)BITS / 8;
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      mbar_arrive_expect_tx(&bar[slot], (unsigned)p_nv * (cbytes + ebytes));
-      bulk_g2s(sp, p_buf0 + coff, cbytes, &bar[slot]);
-      bulk_g2s(sp + 2 * CODE, p_buf0 + ws, ebytes, &bar[slot]);
-      if (p_nv > 1) {
-        bulk_g2s(sp + CODE, p_buf1 + coff, cbytes, &bar[slot]);
-        bulk_g2s(sp + 2 * CODE + expw, p_buf1 + ws, ebytes, &bar[slot]);
-      }
-    }
-    ++issued;
-    p_pos += (std::uint64_t)nr * kRRow;
-    p_rows -= nr;
-  };
-  auto refill = [&]() {
-    if (!ok) return;
-    while (issued < consumed + kRD && p_seek()) p_issue();
-  };
-  __syncthreads(); // s_w of the first item
-
-  const int f = (lane >> 2) & 1; // the lane's chunk swizzle in s_w
-  for (;; ++ck) {
-    refill();
-    const unsigned int id = s_item[ck % 3];
-    if (id >= items) break;
-    const RingItem ci = ring_item(id, groups, vg, m, g.n);
-    const double2* sw2 = reinterpret_cast<const double2*>(s_w) + 2 * lane;
-    for (int u = warp; u < ci.P * ci.C; u += kRW) {
-      const int c = u % ci.C, pair = u / ci.C;
-      const int nv = min(2, ci.G - 2 * pair);
-      const int ra = c * ci.RC, rb = min(ci.rows, ra + ci.RC);
-      double acc0 = 0.0, acc1 = 0.0;
-      for (int r0 = ra; r0 < rb; r0 += R) {
-        const int slot = (int)(consumed % kRD);
-        if (ok && !ring_wait(&bar[slot], (consumed / kRD) & 1u, kLimitNs)) {
-          ok = false;
-          drain_from = consumed;
-          if (lane == 0) {
-            atomicExch(&ctl[1], 1u);
-            s_item[3] = 1u;
-          }
-        }
-        const std::uint8_t* sp = ring + (std::size_t)slot * slot_bytes;
-        const std::uint64_t pos0 = ci.s0 + (std::uint64_t)r0 * kRRow;
-        // exponent offsets in the slot: block of value pos0 + d is
-        // (pos0 >> log2E) + (((pos0 & emask) + d) >> log2E)
-        const int ebase = (int)(((pos0 >> g.log2E) * Wb) & 15u);
-        const int po = (int)(pos0 & (std::uint64_t)emask) + 4 * lane;
-        const int nr = min(R, rb - r0);
+  static_assert((JB & (JB - 1)) == 0 && JB <= 8, "warp_sums");
+  constexpr int Wb = fast_cfg<double, BITS>::W / 8;
+  __shared__ double s_sum[kKW][JB];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
+  const unsigned unit = (blockIdx.x << (3 - lq)) + (unsigned)(warp >> lq);
+  const unsigned sl = unit / groups, gr = unit - sl * groups;
+  const bool live = sl < ns;
+  const int j0 = (int)gr * JB, nv = min(JB, m - j0);
+  double sum = 0.0;
+  if (live) {
+    const unsigned part = S >> lq;
+    const std::uint64_t pos0 = (std::uint64_t)sl * S + (std::uint64_t)(warp & ((1 << lq) - 1)) * part;
+    const int len = pos0 >= g.n ? 0 : (int)min((std::uint64_t)part, g.n - pos0);
+    const bool wvec = (reinterpret_cast<std::uintptr_t>(w) & 31u) == 0;
+    double acc[JB];
 #pragma unroll
-        for (int rr = 0; rr < R; ++rr) {
-          if (rr < nr) {
-            const double2* wr = sw2 + (r0 + rr) * (kRRow / 2);
-            const double2 wa = wr[f], wb = wr[1 - f]; // logical chunks 2 * lane and 2 * lane + 1
-            const double wv[4] = { wa.x, wa.y, wb.x, wb.y };
-            const int eoff = ebase + ((po + rr * kRRow) >> g.log2E) * Wb;
-            lane_words<double, BITS> lw;
-            ring_lane_words<BITS>(sp + rr * RB, lane, lw);
-            lw.be = (typename lane_words<double, BITS>::exp_t)load_exp(sp + 2 * CODE + eoff, S::W);
-            acc0 = lane_dot<BITS>(lw, wv, acc0);
-            if (nv > 1) {
-              lane_words<double, BITS> lw1;
-              ring_lane_words<BITS>(sp + CODE + rr * RB, lane, lw1);
-              lw1.be = (typename lane_words<double, BITS>::exp_t)load_exp(sp + 2 * CODE + expw + eoff, S::W);
-              acc1 = lane_dot<BITS>(lw1, wv, acc1);
-            }
+    for (int jj = 0; jj < JB; ++jj) acc[jj] = 0.0;
+    for (int p = lane * NV; p - lane * NV < len; p += 32 * NV) {
+      const bool in = p < len;
+      const std::uint64_t idx = pos0 + (std::uint64_t)p;
+      const std::uint64_t S0 = idx * (std::uint64_t)BITS;
+      const std::uint64_t eo = (idx >> g.log2E) * Wb;
+      basis_lane<BITS, NV> l[JB];
+#pragma unroll
+      for (int jj = 0; jj < JB; ++jj) {
+        if (in && jj < nv) {
+          const std::uint8_t* buf = bp.buf[j0 + jj];
+          basis_load<BITS, NV>(buf + eo, buf + g.exp_bytes, S0, l[jj]);
+        } else {
+          l[jj].be = 0;
+#pragma unroll
+          for (int i = 0; i < (int)(sizeof(l[jj].w) / 4); ++i) l[jj].w[i] = 0u;
+        }
+      }
+      double wv[NV];
+      if (in && wvec && p + NV <= len) {
+#pragma unroll
+        for (int h = 0; h < NV; h += 4) {
+          std::uint32_t t[8];
+          asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                       : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]),
+                         "=r"(t[7])
+                       : "l"(w + idx + h));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) wv[h + k] = __hiloint2double((int)t[2 * k + 1], (int)t[2 * k]);
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) wv[k] = p + k < len ? __ldg(w + idx + k) : 0.0;
+      }
+      const int o = (int)(S0 & 31u);
+      bool slow = false;
+      if constexpr (has_direct(BITS)) {
+#pragma unroll
+        for (int jj = 0; jj < JB; ++jj) slow |= !direct_exponent<BITS>(l[jj].be);
+        if (!__any_sync(0xFFFFFFFFu, slow)) {
+#pragma unroll
+          for (int jj = 0; jj < JB; ++jj) {
+            double v[NV];
+            basis_values_direct<BITS, NV>(l[jj], o, v);
+            double t = v[0] * wv[0]; // a step's own sum: shorter chains, smaller rounding errors
+#pragma unroll
+            for (int k = 1; k < NV; ++k) t = fma(v[k], wv[k], t);
+            acc[jj] += t;
           }
+        } else if (in) {
+#pragma unroll
+          for (int jj = 0; jj < JB; ++jj)
+            if (jj < nv) {
+              const std::uint8_t* buf = bp.buf[j0 + jj];
+              acc[jj] = slow_lane_dot<BITS, NV, JB>(buf + eo, buf + g.exp_bytes, S0, w + idx, min(NV, len - p), acc[jj]);
+            }
         }
         __syncwarp();
-        ++consumed;
-        refill();
-      }
+      } else {
 #pragma unroll
-      for (int sh = 16; sh > 0; sh >>= 1) {
-        acc0 += __shfl_down_sync(0xFFFFFFFFu, acc0, sh);
-        acc1 += __shfl_down_sync(0xFFFFFFFFu, acc1, sh);
-      }
-      if (lane == 0) {
-        const int t = 2 * pair;
-        s_part[t * ci.C + c] = acc0;
-        if (nv > 1) s_part[(t + 1) * ci.C + c] = acc1;
-      }
-    }
-    // values past the slice's whole warp rows (the array's last, partial row)
-    const bool tail = ci.len > ci.rows * kRRow;
-    if (tail) {
-      const std::uint64_t idx = ci.s0 + (std::uint64_t)ci.rows * kRRow + 4 * (std::uint64_t)lane;
-      const int i = ci.rows * kRRow + 4 * lane;
-      const double2* sw = reinterpret_cast<const double2*>(s_w);
-      const int q0 = i / 2;
-      const double2 wa = sw[q0 ^ ((q0 >> 3) & 1)], wb = sw[(q0 + 1) ^ (((q0 + 1) >> 3) & 1)];
-      const double wv[4] = { wa.x, wa.y, wb.x, wb.y };
-      for (int t = warp; t < ci.G; t += kRW) {
-        double a = 0.0;
-        if (idx < g.n) {
-          const std::uint8_t* buf = bp.buf[ci.jb + t];
-          lane_words<double, BITS> lw;
-          fast_load_lane<double, BITS>(buf, buf + g.exp_bytes, g.log2E, idx, lw);
-          a = lane_dot<BITS>(lw, wv, 0.0);
+        for (int jj = 0; jj < JB; ++jj) {
+          double v[NV];
+          basis_values_any<BITS, NV>(l[jj], o, v);
+          double t = 0.0;
+#pragma unroll
+          for (int k = 0; k < NV; ++k)
+            if (p + k < len) t = fma(v[k], wv[k], t);
+          acc[jj] += t;
         }
-#pragma unroll
-        for (int sh = 16; sh > 0; sh >>= 1) a += __shfl_down_sync(0xFFFFFFFFu, a, sh);
-        if (lane == 0) s_part[kRMaxGroup + t] = a;
       }
     }
-    __syncthreads(); // the item's unit sums are in; s_w is free
-    if (tid < ci.G) {
-      double sum = 0.0;
-      for (int c = 0; c < ci.C; ++c) sum += s_part[tid * ci.C + c];
-      if (tail) sum += s_part[kRMaxGroup + tid];
-      partials[(std::uint64_t)(ci.jb + tid) * ns + ci.s0 / kRSlice] = sum;
-    }
-    if (tid == 0) s_item[(ck + 2) % 3] = atomicAdd(&ctl[0], 1u);
-    const unsigned int nid = s_item[(ck + 1) % 3];
-    if (nid < items) stage_w(nid);
-    __syncthreads(); // next slice of w, item ck + 2 and the abort flag visible
-    if (s_item[3]) break;
+    sum = warp_sums<JB>(acc);
+#pragma unroll
+    for (int sh = 16 / JB; sh > 0; sh >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, sh);
   }
-  // a stop after a wait ran out: let this warp's copies still in flight land
-  // (bounded); after a normal end every issued stage has been consumed
-  if (s_item[3])
-    for (unsigned int q = ok ? consumed : drain_from; q < issued; ++q)
-      ring_wait(&bar[q % kRD], (q / kRD) & 1u, 10000000ull);
+  // lane's sum is vector j0 + lane * JB / 32's
+  const int jj = lane * JB / 32;
+  if (lq == 0) {
+    if (live && lane % (32 / JB) == 0 && jj < nv) partials[(std::uint64_t)(j0 + jj) * ns + sl] = sum;
+    return;
+  }
+  if (lane % (32 / JB) == 0) s_sum[warp][jj] = sum;
+  __syncthreads();
+  if (live && (warp & ((1 << lq) - 1)) == 0 && lane % (32 / JB) == 0 && jj < nv) {
+    for (int q = 1; q < (1 << lq); ++q) sum += s_sum[warp + q][jj];
+    partials[(std::uint64_t)(j0 + jj) * ns + sl] = sum;
+  }
 }
 
 // h[j] = sum over slices of partials[j * ns + slice], in a fixed order; one
-// CTA per vector.  NaN for every h[j] when a ring wait ran out; the last CTA
-// clears the item counter, the error flag and its own ticket for the next call.
+// CTA per vector.
 __global__ void __launch_bounds__(kKT)
-  k_basis_dot_ring_final(const double* __restrict__ partials, unsigned int ns, double* __restrict__ h,
-                         unsigned int* __restrict__ ctl)
+  k_basis_dot_final(const double* __restrict__ partials, unsigned int ns, double* __restrict__ h)
 {
-  __shared__ double s_red[kKT / 32];
+  __shared__ double s_red[kKW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* pj = partials + (std::uint64_t)blockIdx.x * ns;
+  pdl_wait(); // every partial sum is written
   double sum = 0.0;
   for (unsigned int b = tid; b < ns; b += kKT) sum += __ldcg(pj + b);
 #pragma unroll
@@ -759,64 +455,95 @@ __global__ void __launch_bounds__(kKT)
   if (tid == 0) {
     double t = 0.0;
 #pragma unroll
-    for (int q = 0; q < kKT / 32; ++q) t += s_red[q];
-    h[blockIdx.x] = __ldcg(&ctl[1]) ? __longlong_as_double(0x7FF8000000000000ll) : t;
-    __threadfence();
-    if (atomicAdd(&ctl[2], 1u) == gridDim.x - 1) {
-      ctl[0] = 0u;
-      ctl[1] = 0u;
-      ctl[2] = 0u;
-    }
+    for (int q = 0; q < kKW; ++q) t += s_red[q];
+    h[blockIdx.x] = t;
   }
 }
 
-template<int BITS>
-__global__ void __launch_bounds__(kKT, kMinCtas)
+// Bound by DRAM from 24 bits up (0.99-1.06 of the copy bandwidth), by the
+// decode's instructions below (16 bits 0.84, 21 bits 0.73).
+template<int BITS, int NV, int JB>
+__global__ void __launch_bounds__(kKT, axpy_ctas(BITS, NV))
   k_basis_axpy(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ coef,
                double* __restrict__ y)
 {
-  constexpr int P = fast_cfg<double, BITS>::P;
-  constexpr int JB = jb_axpy(BITS);
+  constexpr int Wb = fast_cfg<double, BITS>::W / 8;
   __shared__ double s_c[kMaxBasis];
   for (int j = threadIdx.x; j < m; j += kKT) s_c[j] = __ldg(coef + j);
   __syncthreads();
-  const std::uint64_t stride = (std::uint64_t)gridDim.x * kKT * P;
-  for (std::uint64_t idx = ((std::uint64_t)blockIdx.x * kKT + threadIdx.x) * P; idx < g.n; idx += stride) {
-    const bool whole = idx + P <= g.n;
-    double acc[P];
-    if (whole) {
+  const std::uint64_t idx = ((std::uint64_t)blockIdx.x * kKT + threadIdx.x) * NV;
+  const bool in = idx < g.n, whole = idx + NV <= g.n;
+  double acc[NV];
+  if (whole) {
+#pragma unroll
+    for (int h = 0; h < NV; h += 4) {
       std::uint32_t v[8];
-      ld256_stream(y + idx, v);
+      ld256_stream(y + idx + h, v);
 #pragma unroll
-      for (int k = 0; k < P; ++k) acc[k] = __longlong_as_double(((long long)v[2 * k + 1] << 32) | v[2 * k]);
-    } else {
-#pragma unroll
-      for (int k = 0; k < P; ++k) acc[k] = idx + k < g.n ? y[idx + k] : 0.0;
+      for (int k = 0; k < 4; ++k) acc[h + k] = __hiloint2double((int)v[2 * k + 1], (int)v[2 * k]);
     }
-    for (int j0 = 0; j0 < m; j0 += JB) {
-      lane_words<double, BITS> lw[JB];
+  } else {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) acc[k] = idx + k < g.n ? y[idx + k] : 0.0;
+  }
+  const std::uint64_t S0 = idx * (std::uint64_t)BITS;
+  const std::uint64_t eo = (idx >> g.log2E) * Wb;
+  const int o = (int)(S0 & 31u);
+  for (int j0 = 0; j0 < m; j0 += JB) {
+    basis_lane<BITS, NV> l[JB];
+#pragma unroll
+    for (int jj = 0; jj < JB; ++jj) {
+      l[jj].be = 0;
+      if (in && j0 + jj < m) {
+        const std::uint8_t* buf = bp.buf[j0 + jj];
+        basis_load<BITS, NV>(buf + eo, buf + g.exp_bytes, S0, l[jj]);
+      }
+    }
+    bool slow = false;
+    if constexpr (has_direct(BITS)) {
+#pragma unroll
+      for (int jj = 0; jj < JB; ++jj) slow |= !direct_exponent<BITS>(l[jj].be);
+      slow = __any_sync(0xFFFFFFFFu, slow);
+    }
+    if (!slow) {
 #pragma unroll
       for (int jj = 0; jj < JB; ++jj)
         if (j0 + jj < m) {
-          const std::uint8_t* buf = bp.buf[j0 + jj];
-          fast_load_lane<double, BITS>(buf, buf + g.exp_bytes, g.log2E, idx, lw[jj]);
-        }
+          double v[NV];
+          if constexpr (has_direct(BITS))
+            basis_values_direct<BITS, NV>(l[jj], o, v);
+          else
+            basis_values_any<BITS, NV>(l[jj], o, v);
+          const double cj = s_c[j0 + jj];
 #pragma unroll
-      for (int jj = 0; jj < JB; ++jj)
-        if (j0 + jj < m) lane_axpy<BITS>(lw[jj], s_c[j0 + jj], acc);
+          for (int k = 0; k < NV; ++k) acc[k] = fma(cj, v[k], acc[k]);
+        }
+    } else {
+      if (in) {
+        double t[NV];
+#pragma unroll
+        for (int k = 0; k < NV; ++k) t[k] = acc[k];
+        for (int j = j0; j < min(m, j0 + JB); ++j)
+          slow_lane_axpy<BITS, NV>(bp.buf[j] + eo, bp.buf[j] + g.exp_bytes, S0, s_c[j], t);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) acc[k] = t[k];
+      }
+      __syncwarp();
     }
-    if (whole) {
+  }
+  if (whole) {
+#pragma unroll
+    for (int h = 0; h < NV; h += 4) {
       std::uint32_t v[8];
 #pragma unroll
-      for (int k = 0; k < P; ++k) {
-        const unsigned long long b = (unsigned long long)__double_as_longlong(acc[k]);
-        v[2 * k] = (std::uint32_t)b;
-        v[2 * k + 1] = (std::uint32_t)(b >> 32);
+      for (int k = 0; k < 4; ++k) {
+        v[2 * k] = (std::uint32_t)__double2loint(acc[h + k]);
+        v[2 * k + 1] = (std::uint32_t)__double2hiint(acc[h + k]);
       }
-      st256_stream(y + idx, v);
-    } else {
-      for (int k = 0; k < P && idx + k < g.n; ++k) y[idx + k] = acc[k];
+      st256_stream(y + idx + h, v);
     }
+  } else if (in) {
+    for (int k = 0; k < NV && idx + k < g.n; ++k) y[idx + k] = acc[k];
   }
 }
 
@@ -854,87 +581,79 @@ int basis_args(int dtype, int bits, int E, const void* const* basis, int m, std:
   return FRSZ2_OK;
 }
 
-constexpr int kMaxCtasPerSm = 8; // bound used to size the workspace
+constexpr int kMaxCtasPerSm = 8; // bound that sizes the workspace
 
-// Values per CTA for `ctas` resident CTAs: a multiple of 256 (whole lanes).
-std::uint64_t dot_chunk(std::uint64_t n, std::uint64_t ctas)
+// Launch geometry of the dot.
+struct DotPlan
 {
-  std::uint64_t chunk = (n + ctas - 1) / ctas;
-  return std::max<std::uint64_t>(256, ((chunk + 255) / 256) * 256);
+  unsigned ns, groups, S; // slices, vector groups, positions per slice
+  int lq;                 // log2 of the warps that share a unit
+  unsigned grid;
+};
+
+// A warp walks up to 12 steps of 32 * NV positions (24 measured even), fewer
+// when that would leave fewer than three units for each of the 32 warps that an
+// SM holds.  The workspace has room for max(8 per SM, n / 3072) sums per vector;
+// where short walks would need more, several warps of a CTA share a unit.
+bool dot_plan(int m, std::uint64_t n, int nv, int jb, DotPlan* p)
+{
+  const std::uint64_t rows = std::max<std::uint64_t>((std::uint64_t)sm_count() * kMaxCtasPerSm, (n + kSub - 1) / kSub);
+  const std::uint64_t step = 32 * (std::uint64_t)nv;
+  const std::uint64_t groups = ((std::uint64_t)m + jb - 1) / jb;
+  const std::uint64_t steps = (n + step - 1) / step;
+  const std::uint64_t warps = (std::uint64_t)sm_count() * 32 * 3;
+  std::uint64_t k = std::min<std::uint64_t>(12, std::max<std::uint64_t>(1, (steps * groups + warps - 1) / warps));
+  const std::uint64_t least = (steps + rows - 1) / rows; // steps per slice that the workspace asks for
+  int lq = 0;
+  while (lq < 3 && (k << lq) < least) ++lq;
+  if ((k << lq) < least) k = (least + 7) >> 3;
+  const std::uint64_t S = (k << lq) * step;
+  const std::uint64_t ns = (n + S - 1) / S;
+  const std::uint64_t per = 8u >> lq; // units per CTA
+  const std::uint64_t grid = (ns * groups + per - 1) / per;
+  if (S > 0x7FFFFFFFull || ns * groups > 0xFFFFFFF0ull || grid > 0x7FFFFFFFull) return false;
+  *p = DotPlan{ (unsigned)ns, (unsigned)groups, (unsigned)S, lq, (unsigned)grid };
+  return true;
 }
 
-// axpy grid: up to this many CTAs per SM (about 4 resident), the rest queue
-// and start as others finish; measured on B200, 100 vectors of 2^22 values:
-// 8 per SM 0.871 of HBM, 16 per SM 0.885, one CTA per 1,024 positions 0.887
-// (32 bits; 21 bits 0.516 / 0.545 / 0.542).
-#ifndef FRSZ2_AXPY_CTAS_PER_SM
-#define FRSZ2_AXPY_CTAS_PER_SM 16
-#endif
-
-#ifndef FRSZ2_KRYLOV_DYNAMIC
-#define FRSZ2_KRYLOV_DYNAMIC 1
-#endif
-
-template<int BITS>
-int dyn_ctas_per_sm()
+template<int BITS, int NV, int JB>
+int launch_dot(const BasisParams& bp, int m, const BasisGeo& g, const double* w, double* h, void* workspace,
+               cudaStream_t s)
 {
-  int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_basis_dot_dyn<BITS>, kKT, 0) != cudaSuccess ||
-      blocks < 1)
-    blocks = 1;
-  return std::min(blocks, kMaxCtasPerSm);
-}
-
-template<int BITS>
-int dot_ctas_per_sm()
-{
-  int blocks = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_basis_dot<BITS>, kKT, 0) != cudaSuccess || blocks < 1)
-    blocks = 1;
-  return std::min(blocks, kMaxCtasPerSm);
-}
-
-// Widths whose dot runs on the copy rings.  Measured on B200 (100 vectors of
-// 2^22 values, E 32, of the HBM copy bandwidth; register kernel -> rings):
-// 64 bits 0.78 -> 0.89; 48 bits 0.84 -> 0.65, 32 bits 0.89 -> 0.69, 24 bits
-// 0.68 -> 0.55, 21 bits 0.53 -> 0.46, 16 bits 0.48 -> 0.39.  Below 64 bits a
-// stage holds more values per byte, and the rings' decode, with half the
-// resident warps of the register kernel, falls behind.
-#define FRSZ2_RING_WIDTHS(X) X(64)
-
-// The ring dot: items of up to kRMaxGroup vectors over a slice, one CTA per
-// SM slot the shared memory allows, then the slice-ordered sums.
-template<int BITS>
-int launch_dot_ring(const BasisParams& bp, int m, const BasisGeo& g, const double* w, double* h,
-                    void* workspace, cudaStream_t s)
-{
-  using S = ring_shape<BITS>;
-  const std::uint64_t ns64 = (g.n + kRSlice - 1) / kRSlice;
-  if (ns64 > 0xFFFFFFFFull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
-  const unsigned ns = (unsigned)ns64;
-  const int vg = std::min(m, kRMaxGroup);
-  const std::uint64_t items = ns64 * (std::uint64_t)((m + vg - 1) / vg);
-  if (items > 0xFFFFFFF0ull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
-  const int expw = ring_expw(S::R, g.log2E, S::Wb);
-  const int slot_bytes = (2 * S::CODE + 2 * expw + 127) / 128 * 128;
-  const int smem = ((kRSlice + kRPart) * 8 + kRW * kRD * 8 + 16 + 127) / 128 * 128 + kRW * kRD * slot_bytes;
-  int rc;
-  if ((rc = cuda_status(cudaFuncSetAttribute(k_basis_dot_ring<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             smem),
-                        "dot shared memory")))
-    return rc;
-  int per = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_basis_dot_ring<BITS>, kRT, smem) != cudaSuccess ||
-      per < 1)
-    per = 1;
-  const std::uint64_t ctas = (std::uint64_t)sm_count() * (std::uint64_t)per;
-  const unsigned grid = (unsigned)std::max<std::uint64_t>(1, std::min<std::uint64_t>(items, ctas));
-  auto* ctl = static_cast<unsigned int*>(workspace);
+  DotPlan p;
+  if (!dot_plan(m, g.n, NV, JB, &p)) return set_error(FRSZ2_EFAIL, "basis vectors too long");
   auto* rows = reinterpret_cast<double*>(static_cast<std::uint8_t*>(workspace) + 256);
-  k_basis_dot_ring<BITS><<<grid, kRT, smem, s>>>(bp, m, g, w, ns, vg, expw, slot_bytes, rows, ctl);
-  if ((rc = cuda_status(cudaGetLastError(), "basis dot launch"))) return rc;
-  k_basis_dot_ring_final<<<(unsigned)m, kKT, 0, s>>>(rows, ns, h, ctl);
-  return cuda_status(cudaGetLastError(), "basis dot launch");
+  k_basis_dot<BITS, NV, JB><<<p.grid, kKT, 0, s>>>(bp, m, g, w, p.ns, p.groups, p.S, p.lq, rows);
+  if (int rc = cuda_status(cudaGetLastError(), "basis dot launch")) return rc;
+  // the sums' kernel is set up while the products run and waits for them
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)m);
+  cfg.blockDim = dim3(kKT);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cuda_status(cudaLaunchKernelEx(&cfg, k_basis_dot_final, (const double*)rows, p.ns, h), "basis dot launch");
+}
+
+// The axpy's threads walk the vectors one after the other, so a short array has
+// few of them: below four CTAs per SM of eight values per lane, four per lane
+// (30 vectors of 300,007 values, 32 bits: 14.7 -> 9.9 us; 16 bits 8.5 -> 6.8).
+template<int BITS>
+int launch_axpy(const BasisParams& bp, int m, const BasisGeo& g, const double* coef, double* y, cudaStream_t s)
+{
+  constexpr int NV = basis_nv(BITS), J4 = axpy_jb(BITS, 4), JN = axpy_jb(BITS, NV);
+  const bool four = g.log2E < 3 || (NV == 8 && g.n < (std::uint64_t)sm_count() * 4 * kKT * 8);
+  const std::uint64_t per = (std::uint64_t)kKT * (four ? 4 : NV);
+  const std::uint64_t grid = (g.n + per - 1) / per;
+  if (grid > 0x7FFFFFFFull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
+  if (four)
+    k_basis_axpy<BITS, 4, J4><<<(unsigned)grid, kKT, 0, s>>>(bp, m, g, coef, y);
+  else
+    k_basis_axpy<BITS, NV, JN><<<(unsigned)grid, kKT, 0, s>>>(bp, m, g, coef, y);
+  return cuda_status(cudaGetLastError(), "basis axpy launch");
 }
 
 } // namespace
@@ -967,76 +686,18 @@ int frsz2_basis_dot(int dtype, int bits, int block_size, const void* const* basi
     return set_error(FRSZ2_EFAIL, "workspace must be 256-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (n == 0) return cuda_status(cudaMemsetAsync(h, 0, (std::size_t)m * sizeof(double), s), "memset");
-  switch (bits) {
-#define CASE(B)                                                                                                    \
-  case B: return launch_dot_ring<B>(bp, m, g, static_cast<const double*>(w), static_cast<double*>(h), workspace, s);
-    FRSZ2_RING_WIDTHS(CASE)
-#undef CASE
-    default: break;
-  }
-  if (FRSZ2_KRYLOV_DYNAMIC) {
-    const std::uint64_t ns64 = (n + kSub - 1) / kSub;
-    if (ns64 > 0xFFFFFFFFull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
-    const unsigned ns = (unsigned)ns64;
-    auto* next_slice = static_cast<unsigned int*>(workspace);
-    auto* rows = reinterpret_cast<double*>(static_cast<std::uint8_t*>(workspace) + 256);
-    int per = 1;
-    switch (bits) {
-#define CASE(B)                                                                                                    \
-  case B: per = dyn_ctas_per_sm<B>(); break;
-      FRSZ2_KRYLOV_WIDTHS(CASE)
-#undef CASE
-    }
-    const std::uint64_t ctas = (std::uint64_t)sm_count() * (std::uint64_t)per;
-    // vectors per item: up to 32 vectors, all of them (whole slices); more,
-    // about 8 items per CTA in multiples of jb_dot and at least 16 vectors (each
-    // item stages its slice of w once).  Measured on B200 with 2^22-value
-    // vectors, 32 bits: m = 100 0.76 of HBM with 32 vectors per item against
-    // 0.74 with whole slices; m = 20 0.67 with whole slices against 0.62 with
-    // 16 per item.
-    std::uint64_t vg = (std::uint64_t)m;
-    if (m > 32) {
-      vg = ((std::uint64_t)m * ns + 8 * ctas - 1) / (8 * ctas);
-      const std::uint64_t jb = (std::uint64_t)jb_dot(bits);
-      vg = std::min<std::uint64_t>((std::uint64_t)m, std::max<std::uint64_t>(16, (vg + jb - 1) / jb * jb));
-    }
-    const std::uint64_t items = ns * (((std::uint64_t)m + vg - 1) / vg);
-    if (items > 0xFFFFFFFFull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
-    const unsigned grid = (unsigned)std::max<std::uint64_t>(1, std::min<std::uint64_t>(items, ctas));
-    switch (bits) {
-#define CASE(B)                                                                                                    \
-  case B:                                                                                                          \
-    k_basis_dot_dyn<B><<<grid, kKT, 0, s>>>(bp, m, g, static_cast<const double*>(w), ns, (int)vg, rows,          \
-                                            next_slice);                                                           \
-    break;
-      FRSZ2_KRYLOV_WIDTHS(CASE)
-#undef CASE
-    }
-    if (int rc = cuda_status(cudaGetLastError(), "basis dot launch")) return rc;
-    k_basis_dot_final<<<(unsigned)m, kKT, 0, s>>>(rows, ns, static_cast<double*>(h), next_slice);
-    return cuda_status(cudaGetLastError(), "basis dot launch");
-  }
-  int per_sm = 1;
-  switch (bits) {
-#define CASE(B)                                                                                                    \
-  case B: per_sm = dot_ctas_per_sm<B>(); break;
-    FRSZ2_KRYLOV_WIDTHS(CASE)
-#undef CASE
-  }
-  const std::uint64_t chunk = dot_chunk(n, (std::uint64_t)sm_count() * (std::uint64_t)per_sm);
-  const unsigned grid = (unsigned)std::max<std::uint64_t>(1, (n + chunk - 1) / chunk);
-  auto* ticket = static_cast<unsigned int*>(workspace);
-  auto* partials = reinterpret_cast<double*>(static_cast<std::uint8_t*>(workspace) + 256);
+  const auto* wd = static_cast<const double*>(w);
+  auto* hd = static_cast<double*>(h);
   switch (bits) {
 #define CASE(B)                                                                                                    \
   case B:                                                                                                          \
-    k_basis_dot<B><<<grid, kKT, 0, s>>>(bp, m, g, static_cast<const double*>(w), chunk, partials, ticket,          \
-                                        static_cast<double*>(h));                                                  \
-    break;
+    if (block_size < 8) return launch_dot<B, 4, dot_jb(B)>(bp, m, g, wd, hd, workspace, s);                        \
+    if (m <= 2) return launch_dot<B, basis_nv(B), 2>(bp, m, g, wd, hd, workspace, s);                              \
+    return launch_dot<B, basis_nv(B), dot_jb(B)>(bp, m, g, wd, hd, workspace, s);
     FRSZ2_KRYLOV_WIDTHS(CASE)
 #undef CASE
   }
-  return cuda_status(cudaGetLastError(), "basis dot launch");
+  return FRSZ2_EFAIL;
 }
 
 int frsz2_basis_axpy(int dtype, int bits, int block_size, const void* const* basis, int m, uint64_t n,
@@ -1050,18 +711,15 @@ int frsz2_basis_axpy(int dtype, int bits, int block_size, const void* const* bas
   if (!coef || !y) return set_error(FRSZ2_EFAIL, "null pointer");
   if (reinterpret_cast<std::uintptr_t>(y) % 32 != 0) return set_error(FRSZ2_EFAIL, "y must be 32-byte aligned");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const std::uint64_t lanes = (n + 3) / 4;
-  const unsigned grid = (unsigned)std::max<std::uint64_t>(
-    1, std::min<std::uint64_t>((lanes + kKT - 1) / kKT, (std::uint64_t)sm_count() * FRSZ2_AXPY_CTAS_PER_SM));
+  const auto* cd = static_cast<const double*>(coef);
+  auto* yd = static_cast<double*>(y);
   switch (bits) {
 #define CASE(B)                                                                                                    \
-  case B:                                                                                                          \
-    k_basis_axpy<B><<<grid, kKT, 0, s>>>(bp, m, g, static_cast<const double*>(coef), static_cast<double*>(y));     \
-    break;
+  case B: return launch_axpy<B>(bp, m, g, cd, yd, s);
     FRSZ2_KRYLOV_WIDTHS(CASE)
 #undef CASE
   }
-  return cuda_status(cudaGetLastError(), "basis axpy launch");
+  return FRSZ2_EFAIL;
 }
 
 } // extern "C"
