@@ -380,6 +380,45 @@ __device__ __forceinline__ typename fp<T>::U decode_plain(typename fast_cfg<T, B
   return r | ((U)(code >> (BITS - 1)) << (fp<T>::UBITS - 1));
 }
 
+// ---------------------------------------------------------------- block maxima
+
+// Largest raw key (key_of<T>::raw) of N values, with floating-point maxima of
+// three magnitudes per instruction: the keys of finite values are positive
+// floats (fp32) or, as the high words of doubles, order like them.  A NaN comes
+// out as the canonical NaN's bits, which are above SPECIAL, and so does a double
+// whose high word reads as a float NaN (|x| >= 2^1017): such a block takes the
+// integer arithmetic, which is exact for it too.
+__device__ __forceinline__ float max3_abs(float a, float b, float c)
+{
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+template<class T, int N, int FROM, int P>
+__device__ __forceinline__ std::uint32_t raw_max(const typename fp<T>::U (&u)[P])
+{
+  float v[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) v[i] = __uint_as_float((std::uint32_t)(sizeof(T) == 4 ? u[FROM + i] : u[FROM + i] >> (fp<T>::UBITS - 32)));
+  if constexpr (N == 1) {
+    return key_of<T>::raw(u[FROM]);
+  } else {
+    float m = max3_abs(v[0], v[1], v[N > 2 ? 2 : 1]);
+#pragma unroll
+    for (int i = 3; i < N; i += 2) m = max3_abs(m, v[i], v[i + 1 < N ? i + 1 : i]);
+    return __float_as_uint(m);
+  }
+}
+
+// Half lanes of fp32 at 24 bits: the float maxima cost registers there (E 20 0.83
+// of HBM with integer ones and no register cap, 0.55 with float ones, 0.82 capped).
+template<class T, int BITS>
+__host__ __device__ constexpr bool half_keeps_integer_max()
+{
+  return sizeof(T) == 4 && BITS == 24;
+}
+
 // ---------------------------------------------------------------- compress
 
 #ifndef FRSZ2_STAGE_NW_MASK
@@ -553,9 +592,14 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
         const int t = ((rr * Cfg::WARPS + warp) * 32 + lane) * 2;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          std::uint32_t m = K::raw(u[rr][h * H]);
+          std::uint32_t m;
+          if constexpr (half_keeps_integer_max<T, BITS>()) {
+            m = K::raw(u[rr][h * H]);
 #pragma unroll
-          for (int i = 1; i < H; ++i) m = max(m, K::raw(u[rr][h * H + i]));
+            for (int i = 1; i < H; ++i) m = max(m, K::raw(u[rr][h * H + i]));
+          } else {
+            m = h == 0 ? raw_max<T, H, 0>(u[rr]) : raw_max<T, H, H>(u[rr]);
+          }
           std::uint32_t cm = m;
           if (m >= K::SPECIAL) {
             cm = K::clean(u[rr][h * H]);
@@ -591,9 +635,7 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
     bool any_special = false;
 #pragma unroll
     for (int rr = 0; rr < RPW; ++rr) {
-      std::uint32_t m = K::raw(u[rr][0]);
-#pragma unroll
-      for (int i = 1; i < P; ++i) m = max(m, K::raw(u[rr][i]));
+      const std::uint32_t m = raw_max<T, P, 0>(u[rr]);
       km[rr] = m;
       any_special |= m >= K::SPECIAL;
     }
@@ -736,11 +778,11 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
         }
       } else if constexpr (ESM == 0) {
         const int field = (int)(kc[rr] >> K::FSHIFT);
-        const std::int64_t ex = exponent_of_field<T>(field);
-        const std::int64_t be = wrap_signed(ex, W);
-        const bool plain = km[rr] < K::SPECIAL && be == ex && plain_exponent<T>(be);
+        const int ex = exponent_of_field<T>(field);
+        const int be = W == 8 && sizeof(T) == 8 ? (int)(std::int8_t)ex : ex; // the other widths hold every exponent
+        const bool plain = km[rr] < K::SPECIAL && be == ex && be >= (sizeof(T) == 4 ? -95 : -959);
         if (plain) {
-          const T scale = pow2<T>(BITS - 2 - (int)be);
+          const T scale = pow2<T>(BITS - 2 - be);
 #pragma unroll
           for (int i = 0; i < P; ++i) c[i] = encode_plain<T, BITS>(u[rr][i], scale);
         } else {
@@ -748,7 +790,7 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
           for (int i = 0; i < P; ++i) c[i] = (C)to_code<T>(u[rr][i], (std::int16_t)be, BITS);
         }
         if ((GEN ? idx == bl * E : (idx & (E - 1)) == 0) && bl < nbt)
-          store_word(j.exps + (b0 + (std::uint64_t)bl) * (std::uint64_t)(W / 8), (std::uint64_t)be, W);
+          store_word(j.exps + (b0 + (std::uint64_t)bl) * (std::uint64_t)(W / 8), (std::uint64_t)(std::int64_t)be, W);
       } else {
         // the lane's P / ESM blocks, each with its own exponent
         constexpr int NBL = P / ESM;
@@ -894,9 +936,42 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
   }
 }
 
+// CTAs of 256 threads per SM that a compress instance's register budget must
+// allow (0: ptxas's choice).  The loads of more tiles in flight are worth more
+// than the registers up to about 16 bits (fp32) / 30 bits (fp64), where ptxas
+// takes 47-58 registers by itself; padded blocks and wider segments spill under
+// a cap.  Measured on B200, 2^27 fp32 / 2^26 fp64 values, E 64 unless given, of
+// the copy bandwidth with no cap / 5 / 6 / 8 CTAs:
+//   fp32  4 bits 0.97 / 0.94 / 1.00 / 1.06, 6 0.82 / 0.90 / 0.93 / 0.95, 13 0.88 /
+//         0.93 / 1.00 / 1.05, 16 1.06 / 1.04 / 1.08 / 1.05, 17 1.02 / 0.94 / 0.97 /
+//         0.94, 21 1.04 / 0.97 / 1.01 / 0.96, 24 1.01 / 1.07 / 1.05 / 1.04
+//   fp64  5 bits 0.92 / 0.91 / 0.94 / 0.99, 13 0.98 / 0.96 / 0.99 / 1.00, 21 1.00 /
+//         0.98 / 1.02 / 1.06, 24 1.09 / 1.04 / 1.09 / 1.06, 30 1.03 / 1.01 / 1.05 /
+//         1.05, 33 1.04 / 0.96 / 1.00 / 0.97
+//   padded blocks (13 bits, E 8): fp32 0.98 / 0.86 / 0.86 / 0.84
+//   values off the 32-byte layout by one: fp32 16 bits 0.77 / 0.85 / 0.93 / 1.00,
+//         fp64 32 bits 0.88 / 0.88 / 0.94 / 1.02
+//   whole-block tiles (GEN): fp32 16 bits E 24 0.96 / 0.88 / 0.93 / 1.03, 32 bits
+//         E 24 0.91 / 1.00 / 1.05 / 1.03, E 20 0.62 / 0.84 / 0.90 / 0.90; fp64 16
+//         bits E 48 0.92 / 0.82 / 0.91 / 0.96, 48 bits E 24 0.94 / 0.93 / 1.02 / 1.00
+//   blocks below a lane: fp32 16 bits E 2 0.88 / 0.94 / 0.94 / 0.92, E 4 24 bits
+//         1.03 / 1.05 / 1.04 / 1.04; fp64 16 bits E 2 0.98 / 1.00 / 1.03 / 0.99
+template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
+__host__ __device__ constexpr int compress_ctas()
+{
+  constexpr bool F32 = sizeof(T) == 4;
+  if (PAD) return 0;
+  if (HALF && half_keeps_integer_max<T, BITS>()) return 0;
+  if (ESM) return F32 ? (BITS <= 16 ? 6 : ESM == 4 && BITS <= 24 ? 5 : 0) : (BITS > 8 && BITS <= 32 ? 6 : 0);
+  if (GEN) return BITS > 32 || (F32 && BITS == 32) ? 6 : 8;
+  if (MIS) return 8;
+  if (F32) return BITS <= 15 ? 8 : BITS == 16 ? 6 : BITS == 24 ? 5 : 0;
+  return BITS <= 30 && BITS != 24 ? 8 : 0;
+}
+
 template<class T, int BITS, int NT = kNT, int RPW = 2, bool PAD = false, int ESM = 0, bool MIS = false,
          bool GEN = false, bool HALF = false, bool WCR = false>
-__global__ void __launch_bounds__(NT) k_compress_fast(Job j)
+__global__ void __launch_bounds__(NT, compress_ctas<T, BITS, PAD, ESM, MIS, GEN, HALF>()) k_compress_fast(Job j)
 {
   __shared__ std::uint32_t s_rmax[2 * fast_cfg<T, BITS, NT, RPW>::ROWS];
   __shared__ __align__(16) std::uint32_t s_stage[stage_words<T, BITS, NT, RPW, ESM>::value];
