@@ -248,6 +248,31 @@ int launch_decompress(const Job& j, int dtype, cudaStream_t s, bool* used_tile)
                               : launch_decompress_t<double>(j, dtype, s, used_tile);
 }
 
+template<class T>
+static void launch_elements_t(const Job& j, const std::uint64_t* idx, std::uint64_t count, T* out, cudaStream_t s)
+{
+  const unsigned grid = grid_for(count, kNT);
+  const std::uint64_t mE = j.log2E < 0 ? ~0ull / (std::uint64_t)j.E + 1 : 0; // E not a power of two
+  switch (j.W) {
+    case 8: k_decompress_elements<T, 8><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
+    case 16: k_decompress_elements<T, 16><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
+    case 32: k_decompress_elements<T, 32><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
+    default:
+      if constexpr (sizeof(T) == 8) k_decompress_elements<T, 64><<<grid, kNT, 0, s>>>(j, mE, idx, count, out);
+  }
+}
+
+// Enqueue the decode of the values at `count` indices.
+static int launch_elements(const Job& j, int dtype, const std::uint64_t* idx, std::uint64_t count, void* out,
+                           cudaStream_t s)
+{
+  if (dtype == FRSZ2_FLOAT)
+    launch_elements_t<float>(j, idx, count, static_cast<float*>(out), s);
+  else
+    launch_elements_t<double>(j, idx, count, static_cast<double*>(out), s);
+  return cuda_status(cudaGetLastError(), "element decode launch");
+}
+
 static int check_alignment(int dtype, const Layout& L, const void* values, const void* buf)
 {
   const std::size_t es = dtype == FRSZ2_FLOAT ? 4 : 8;
@@ -543,12 +568,7 @@ int frsz2_decompress_elements(int dtype, int bits, int block_size, const void* d
   Job j = job_for_slice(L, dtype, 0, L.nb, nullptr, nullptr,
                         const_cast<std::uint8_t*>(static_cast<const std::uint8_t*>(d_compressed)));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const unsigned grid = grid_for(count, kNT);
-  if (dtype == FRSZ2_FLOAT)
-    k_decompress_elements<float><<<grid, kNT, 0, s>>>(j, d_idx, count, static_cast<float*>(d_out));
-  else
-    k_decompress_elements<double><<<grid, kNT, 0, s>>>(j, d_idx, count, static_cast<double*>(d_out));
-  return cuda_status(cudaGetLastError(), "element decode launch");
+  return launch_elements(j, dtype, d_idx, count, d_out, s);
 }
 
 // Host-buffer random access (decompress_cpu_element, include/frsz2.hpp:1199-1214):
@@ -611,12 +631,7 @@ int frsz2_decompress_elements_host(int dtype, int bits, int block_size, const vo
       (rc = cuda_status(cudaMemcpyAsync(S.d_values, h_out, count * es, cudaMemcpyHostToDevice, s), "H2D")))
     return rc;
   Job j = job_for_slice(M, dtype, 0, M.nb, nullptr, nullptr, d_buf);
-  const unsigned grid = grid_for(count, kNT);
-  if (dtype == FRSZ2_FLOAT)
-    k_decompress_elements<float><<<grid, kNT, 0, s>>>(j, d_idx, count, static_cast<float*>(S.d_values));
-  else
-    k_decompress_elements<double><<<grid, kNT, 0, s>>>(j, d_idx, count, static_cast<double*>(S.d_values));
-  if ((rc = cuda_status(cudaGetLastError(), "element decode launch"))) return rc;
+  if ((rc = launch_elements(j, dtype, d_idx, count, S.d_values, s))) return rc;
   if ((rc = cuda_status(cudaMemcpyAsync(h_out, S.d_values, count * es, cudaMemcpyDeviceToHost, s), "D2H"))) return rc;
   return cuda_status(cudaStreamSynchronize(s), "stream synchronize");
 }

@@ -543,33 +543,41 @@ __global__ void __launch_bounds__(kNT) k_decompress_tile(Job j)
 
 namespace frsz2b {
 
-// Random access decode (decompress_cpu_element, frsz2.hpp:1199-1214): one
+// ---------------------------------------------------------------- elements
+
+// Random access (decompress_cpu_element, include/frsz2.hpp:1199-1214): one
 // thread per requested index; indices >= n decode nothing and write nothing.
-template<class T>
-__global__ void __launch_bounds__(kNT)
-  k_decompress_elements(Job j, const std::uint64_t* __restrict__ idx, std::uint64_t count, T* __restrict__ out)
+//
+// Bound by scattered DRAM accesses: every element fetches its word's sector (64
+// bytes of DRAM) and, mostly from L2, its exponent's.  Positions take a shift or
+// one multiply-high (mE = floor(2^64 / E) + 1, exact for g * E < 2^64) instead of
+// three 64-bit divisions, and the word width is a template parameter.  Measured
+// on B200, 2^20 indices into 2^26 fp32 values at 16 bits, E 32: 19.0 -> 18.3 us;
+// 4,000,003 into 2^24 fp64 values, E 5: 51.9 -> 45.5; 1,000 indices 2.41 -> 2.21.
+// 2, 4 or 8 indices per thread, all their loads issued first, took 18.4, 19.2 and
+// 20.5 us: more loads in flight do not help.
+template<class T, int W>
+__global__ void __launch_bounds__(kNT) k_decompress_elements(Job j, std::uint64_t mE,
+                                                             const std::uint64_t* __restrict__ idx,
+                                                             std::uint64_t count, T* __restrict__ out)
 {
   using U = typename fp<T>::U;
-  const int bits = j.bits, W = j.W;
-  const std::uint64_t wmask = W == 64 ? ~0ull : ((1ull << W) - 1);
-  for (std::uint64_t t = (std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < count;
-       t += (std::uint64_t)gridDim.x * blockDim.x) {
-    const std::uint64_t g = idx[t];
+  using word = std::conditional_t<W == 8, std::uint8_t,
+                                  std::conditional_t<W == 16, std::uint16_t,
+                                                     std::conditional_t<W == 32, std::uint32_t, unsigned long long>>>;
+  const int bits = j.bits;
+  for (std::uint64_t t = (std::uint64_t)blockIdx.x * kNT + threadIdx.x; t < count;
+       t += (std::uint64_t)gridDim.x * kNT) {
+    const std::uint64_t g = __ldg(idx + t);
     if (g >= j.n) continue;
-    const std::uint64_t b = g / (std::uint64_t)j.E;
-    const int k = (int)(g - b * (std::uint64_t)j.E);
-    const std::int64_t be = load_exp(j.exps + b * (std::uint64_t)(W / 8), W);
-    const std::uint8_t* wbase = j.words + b * (std::uint64_t)j.block_bytes;
-    const std::int64_t p = (std::int64_t)k * bits;
-    const std::int64_t w = p / W;
-    const int o = (int)(p - w * W);
-    std::uint64_t res = load_word(wbase + w * (W / 8), W);
-    if (W != bits) {
-      res >>= o;
-      if (o + bits > W) res |= load_word(wbase + (w + 1) * (W / 8), W) << (W - o);
-      res &= wmask;
-    }
-    out[t] = from_code<T>((U)res, be, bits);
+    const std::uint64_t b = j.log2E >= 0 ? g >> j.log2E : __umul64hi(g, mE);
+    const std::uint32_t p = (std::uint32_t)(g - b * (std::uint64_t)j.E) * (std::uint32_t)bits;
+    const word* w = reinterpret_cast<const word*>(j.words + b * (std::uint64_t)j.block_bytes) + p / W;
+    const int o = (int)(p % W);
+    const word e = __ldg(reinterpret_cast<const word*>(j.exps) + b);
+    std::uint64_t c = (std::uint64_t)__ldg(w) >> o; // from_code drops the bits above the code's
+    if (o + bits > W) c |= (std::uint64_t)__ldg(w + 1) << (W - o);
+    out[t] = from_code<T>((U)c, (std::int64_t)(std::make_signed_t<word>)e, bits);
   }
 }
 
