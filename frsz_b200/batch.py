@@ -11,7 +11,7 @@ from typing import List, Optional, Sequence
 import torch
 
 from ._lib import BatchItemC, BatchStatsC, check, lib
-from .codec import dtype_code
+from .codec import _stream_ptr, dtype_code
 
 
 @dataclass
@@ -52,7 +52,7 @@ class BatchPlan:
         self._h = h
 
     def _stream(self, stream):
-        return (stream or torch.cuda.current_stream()).cuda_stream
+        return _stream_ptr(stream)
 
     def compress(self, stream: Optional[torch.cuda.Stream] = None) -> None:
         check(lib().frsz2_batch_compress(self._h, self._stream(stream)))
