@@ -16,6 +16,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace frsz2b {
@@ -302,9 +303,30 @@ Job job_for_slice(const Layout& L, int dtype, std::uint64_t b0, std::uint64_t nb
 
 namespace {
 
+// One worker's place in the staged host path: pinned and device buffers of a
+// slice each way, and a stream.
+struct HostSlot
+{
+  std::uint8_t* pin[2] = { nullptr, nullptr }; // into the device, out of it
+  std::uint8_t* dev[2] = { nullptr, nullptr };
+  cudaStream_t st = nullptr;
+};
+
+// Workers of the staged path at most, and the slice of values each takes at a
+// time.  A slice's compressed form has at most twice its bytes (blocks of one
+// value), which sizes a slot's four buffers: 48 MiB pinned and 48 MiB of device
+// memory for all slots, allocated as calls first need them and kept.  Measured
+// with 16 host threads, 2^23 fp64 values at 32 bits, compress / decompress (ms):
+// 8 workers 4.6 / 3.1, 12 3.8 / 2.7, 15 4.0 / 2.7; 12 with slices of 256 KiB
+// 5.2 / 3.8, 512 KiB 4.8 / 3.2, 2 MiB 3.8 / 2.7.
+constexpr int kHostWorkers = 12;
+constexpr std::size_t kHostSlice = (std::size_t)1 << 20;
+constexpr std::size_t kHostSlot = 2 * kHostSlice + 4096;
+
 struct Staging
 {
   std::mutex mu;
+  HostSlot slot[kHostWorkers];
   void* d_values = nullptr;
   std::size_t values_cap = 0;
   void* d_buf = nullptr;
@@ -361,6 +383,136 @@ std::uint64_t slice_blocks(const Layout& L, int dtype)
   return blocks;
 }
 
+int slot_init(HostSlot& h)
+{
+  int rc;
+  for (int d = 0; d < 2; ++d) {
+    if (!h.pin[d] &&
+        (rc = cuda_status(cudaHostAlloc(reinterpret_cast<void**>(&h.pin[d]), kHostSlot, cudaHostAllocDefault),
+                          "staging allocation")))
+      return rc;
+    if (!h.dev[d] && (rc = cuda_status(cudaMalloc(reinterpret_cast<void**>(&h.dev[d]), kHostSlot), "staging allocation")))
+      return rc;
+  }
+  if (!h.st) return cuda_status(cudaStreamCreateWithFlags(&h.st, cudaStreamNonBlocking), "stream create");
+  return FRSZ2_OK;
+}
+
+// Ordinary host memory, pinned host memory, or neither (device, managed).
+enum class Memory { pageable, pinned, other };
+Memory memory_of(const void* p)
+{
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return Memory::other;
+  }
+  return a.type == cudaMemoryTypeUnregistered ? Memory::pageable
+         : a.type == cudaMemoryTypeHost       ? Memory::pinned
+                                              : Memory::other;
+}
+
+// The host path for ordinary (pageable) memory.  A copy between pageable
+// memory and the device goes through the driver's own staging on the calling
+// thread, one copy at a time (10 GB/s for a compress and decompress of 64 MiB);
+// here several threads each take a slice at a time through a pinned slot of
+// their own -- copy in, transfer, kernel, transfer, copy out -- so the copies of
+// some overlap the transfers of others.  The threads live as long as the call; an
+// array of one slice needs none.  Measured with 16 host threads, fp64 at 32 bits,
+// compress / decompress: 2^23 values 14.1 / 6.6 -> 3.8 / 2.7 ms, 2^20 1.11 / 0.92 ->
+// 0.82 / 0.60 ms, 300,001 (slices of 512 KiB up to 8 MiB; of 1 MiB 0.42 / 0.48) 0.42
+// / 0.35 -> 0.30 / 0.25 ms, 4,096 69 / 57 -> 43 / 48 us.
+// Returns false when no slot could be had; the caller then copies directly.
+bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, const std::uint8_t* in,
+                       std::uint8_t* out, int dev, int* result)
+{
+  const std::size_t es = dtype == FRSZ2_FLOAT ? 4 : 8, wb = (std::size_t)L.W / 8;
+  const std::uint64_t bytes = L.n * es;
+  const std::size_t want = bytes > kHostSlice && bytes <= 8 * kHostSlice ? kHostSlice / 2 : kHostSlice;
+  const std::uint64_t per = std::max<std::uint64_t>(1, want / ((std::uint64_t)L.E * es)); // blocks per slice
+  const std::uint64_t slices = (L.nb + per - 1) / per;
+  const unsigned hw = std::thread::hardware_concurrency();
+  const int wanted = (int)std::min<std::uint64_t>(
+    slices, (std::uint64_t)std::min<unsigned>(kHostWorkers, std::max(1u, hw ? hw - hw / 4 : 1u)));
+  int workers = 0;
+  while (workers < wanted && slot_init(S.slot[workers]) == FRSZ2_OK) ++workers;
+  if (workers == 0) return false;
+
+  std::atomic<std::uint64_t> next{ 0 };
+  std::atomic<int> status{ FRSZ2_OK };
+  std::mutex err_mu;
+  std::string err;
+  auto slice = [&](HostSlot& h, std::uint64_t k) -> int {
+    const std::uint64_t b0 = k * per, nbk = std::min(per, L.nb - b0);
+    const std::uint64_t e0 = b0 * (std::uint64_t)L.E;
+    const std::uint64_t ne = std::min<std::uint64_t>(L.n - e0, nbk * (std::uint64_t)L.E);
+    const std::size_t exp_len = nbk * wb, w_at = (exp_len + 255) / 256 * 256; // exponents, then words, in a slot
+    const std::size_t w_len = nbk * (std::size_t)L.block_bytes;
+    const std::uint64_t exp_off = b0 * wb, w_off = L.exp_bytes + b0 * (std::uint64_t)L.block_bytes;
+    Layout P = L;
+    P.n = ne;
+    Job j = make_job(P, dtype);
+    int rc;
+    if (compress) {
+      j.values_in = h.dev[0];
+      j.exps = h.dev[1];
+      j.words = h.dev[1] + w_at;
+      // only the bytes the reference writes go to the caller: of a partial last
+      // block, the words its values reach
+      const std::size_t out_len = w_len - L.block_bytes +
+                                  written_block_bytes((int)(ne - (nbk - 1) * (std::uint64_t)L.E), L.bits, L.W);
+      std::memcpy(h.pin[0], in + e0 * es, ne * es);
+      if ((rc = cuda_status(cudaMemcpyAsync(h.dev[0], h.pin[0], ne * es, cudaMemcpyHostToDevice, h.st), "H2D")) ||
+          (rc = launch_compress(j, dtype, h.st, nullptr)) ||
+          (rc = cuda_status(cudaMemcpyAsync(h.pin[1], h.dev[1], w_at + out_len, cudaMemcpyDeviceToHost, h.st),
+                            "D2H")) ||
+          (rc = cuda_status(cudaStreamSynchronize(h.st), "stream sync")))
+        return rc;
+      std::memcpy(out + exp_off, h.pin[1], exp_len);
+      std::memcpy(out + w_off, h.pin[1] + w_at, out_len);
+    } else {
+      j.exps = h.dev[0];
+      j.words = h.dev[0] + w_at;
+      j.values_out = h.dev[1];
+      std::memcpy(h.pin[0], in + exp_off, exp_len);
+      std::memcpy(h.pin[0] + w_at, in + w_off, w_len);
+      if ((rc = cuda_status(cudaMemcpyAsync(h.dev[0], h.pin[0], w_at + w_len, cudaMemcpyHostToDevice, h.st), "H2D")) ||
+          (rc = launch_decompress(j, dtype, h.st, nullptr)) ||
+          (rc = cuda_status(cudaMemcpyAsync(h.pin[1], h.dev[1], ne * es, cudaMemcpyDeviceToHost, h.st), "D2H")) ||
+          (rc = cuda_status(cudaStreamSynchronize(h.st), "stream sync")))
+        return rc;
+      std::memcpy(out + e0 * es, h.pin[1], ne * es);
+    }
+    return FRSZ2_OK;
+  };
+  auto work = [&](int w) {
+    int rc = w == 0 ? FRSZ2_OK : cuda_status(cudaSetDevice(dev), "cudaSetDevice");
+    if (!rc) rc = cuda_status(cudaStreamWaitEvent(S.slot[w].st, S.ev_start, 0), "stream wait");
+    for (std::uint64_t k; !rc && status.load(std::memory_order_relaxed) == FRSZ2_OK &&
+                          (k = next.fetch_add(1, std::memory_order_relaxed)) < slices;)
+      rc = slice(S.slot[w], k);
+    if (rc) {
+      cudaStreamSynchronize(S.slot[w].st); // nothing of this call stays in flight
+      std::lock_guard<std::mutex> g(err_mu);
+      if (status.load() == FRSZ2_OK) {
+        err = last_error(); // this thread's
+        status.store(rc);
+      }
+    }
+  };
+  std::vector<std::thread> threads;
+  try {
+    threads.reserve((std::size_t)workers);
+    for (int w = 1; w < workers; ++w) threads.emplace_back(work, w);
+  } catch (...) {
+    // no more threads to be had: those there are and this one take all the slices
+  }
+  work(0);
+  for (auto& t : threads) t.join();
+  *result = status.load() == FRSZ2_OK ? FRSZ2_OK : set_error(status.load(), err);
+  return true;
+}
+
 } // namespace
 
 int host_codec(bool compress, int dtype, int bits, int E, const void* h_in, std::uint64_t n, void* h_out,
@@ -379,14 +531,24 @@ int host_codec(bool compress, int dtype, int bits, int E, const void* h_in, std:
   std::lock_guard<std::mutex> lock(S.mu);
   if ((rc = staging_init(S))) return rc;
   const std::size_t es = dtype == FRSZ2_FLOAT ? 4 : 8;
-  if ((rc = ensure(&S.d_values, &S.values_cap, L.n * es))) return rc;
-  if ((rc = ensure(&S.d_buf, &S.buf_cap, L.total_bytes))) return rc;
-  std::uint8_t* d_buf = static_cast<std::uint8_t*>(S.d_buf);
   const std::uint8_t* hb_in = static_cast<const std::uint8_t*>(h_in);
   std::uint8_t* hb_out = static_cast<std::uint8_t*>(h_out);
 
   // order after prior work on the caller's stream
   if ((rc = cuda_status(cudaEventRecord(S.ev_start, user), "event record"))) return rc;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(user, &cap) != cudaSuccess) cudaGetLastError();
+  // buffers pinned on both sides transfer directly, and what is not host memory,
+  // or a capturing stream, keeps that path's refusal
+  const Memory mi = memory_of(h_in), mo = memory_of(h_out);
+  if (cap == cudaStreamCaptureStatusNone && mi != Memory::other && mo != Memory::other &&
+      (mi == Memory::pageable || mo == Memory::pageable) &&
+      host_codec_staged(S, compress, dtype, L, hb_in, hb_out, dev, &rc))
+    return rc;
+
+  if ((rc = ensure(&S.d_values, &S.values_cap, L.n * es))) return rc;
+  if ((rc = ensure(&S.d_buf, &S.buf_cap, L.total_bytes))) return rc;
+  std::uint8_t* d_buf = static_cast<std::uint8_t*>(S.d_buf);
   for (auto& s : S.st)
     if ((rc = cuda_status(cudaStreamWaitEvent(s, S.ev_start, 0), "stream wait"))) return rc;
 

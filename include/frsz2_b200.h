@@ -89,7 +89,10 @@ int frsz2_decompress(int dtype, int bits, int block_size, const void* d_compress
 /* Host buffers: the same codec with the host<->device copies inside the call
  * (pinned memory recommended; pageable works).  Synchronous: returns when the
  * result is in host memory.  This is the drop-in for the reference's host-side
- * compress_cpu_impl / decompress_cpu_impl calls. */
+ * compress_cpu_impl / decompress_cpu_impl calls.  Ordinary memory goes through pinned slots
+ * (up to 48 MiB pinned and 48 MiB of device memory per device, kept) by up to
+ * 12 threads that end with the call, three quarters of the host's cores at
+ * most; pinned buffers transfer directly. */
 int frsz2_compress_host(int dtype, int bits, int block_size, const void* h_values, uint64_t n, void* h_compressed,
                         void* stream);
 int frsz2_decompress_host(int dtype, int bits, int block_size, const void* h_compressed, uint64_t n, void* h_values,
