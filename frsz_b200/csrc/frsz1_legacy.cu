@@ -144,6 +144,7 @@ template<class T>
 __global__ void __launch_bounds__(256) k_frsz1_compress(const T* __restrict__ x, std::uint64_t n, double inv,
                                                         std::int16_t* __restrict__ out, bool vec)
 {
+  enter_in_stream_order();
   static_assert(kComV * 32 == kLegacyBlock, "one block per warp");
   constexpr int V = kComV;
   const int lane = threadIdx.x & 31;
@@ -289,6 +290,7 @@ template<class T, bool OWN, bool RND>
 __global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t* __restrict__ in, std::uint64_t n,
                                                              double ebx2, T* __restrict__ y)
 {
+  enter_in_stream_order();
   constexpr int VO = 64;                        // values per block and part
   constexpr int CS = sizeof(T) == 4 ? 64 : 128; // codes per block and stage
   constexpr int kOutBytes = VO * (int)sizeof(T);
@@ -392,6 +394,7 @@ template<class T, bool OWN>
 __global__ void __launch_bounds__(kDecBlocks) k_frsz1_decompress(const std::int16_t* __restrict__ in, std::uint64_t n,
                                                                   double ebx2, T* __restrict__ y, bool vec)
 {
+  enter_in_stream_order();
   // block 0's differences (the reference reads them for every block)
   __shared__ std::int16_t s_d0[OWN ? 1 : kLegacyBlock];
   __shared__ T s_out[kDecBlocks][kDecChunk + 1];
@@ -470,8 +473,8 @@ int legacy_compress(double eps, const void* d_values, std::uint64_t n, void* d_o
                    reinterpret_cast<std::uintptr_t>(d_out) % 8 == 0;
   const std::uint64_t threads = (n + kComV - 1) / kComV;
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, (threads + 255) / 256);
-  k_frsz1_compress<T><<<grid, 256, 0, s>>>(static_cast<const T*>(d_values), n, 1.0 / (eps * 2.0),
-                                          static_cast<std::int16_t*>(d_out), vec);
+  launch(k_frsz1_compress<T>, grid, 256, 0, s, static_cast<const T*>(d_values), n, 1.0 / (eps * 2.0),
+         static_cast<std::int16_t*>(d_out), vec);
   return cuda_status(cudaGetLastError(), "legacy compress launch");
 }
 
@@ -490,18 +493,18 @@ int legacy_decompress(double eps, const void* d_in, std::uint64_t n, void* d_val
     const unsigned warps = (unsigned)std::max<std::uint64_t>(1, (nb + 31) / 32);
     const bool rnd = sizeof(T) == 4 && s2 >= 0x1p-64 && s2 <= 0x1p96;
     if (own)
-      rnd ? k_frsz1_decompress_vec<T, true, true><<<warps, 32, 0, s>>>(q, n, s2, y)
-          : k_frsz1_decompress_vec<T, true, false><<<warps, 32, 0, s>>>(q, n, s2, y);
+      rnd ? launch(k_frsz1_decompress_vec<T, true, true>, warps, 32, 0, s, q, n, s2, y)
+          : launch(k_frsz1_decompress_vec<T, true, false>, warps, 32, 0, s, q, n, s2, y);
     else
-      rnd ? k_frsz1_decompress_vec<T, false, true><<<warps, 32, 0, s>>>(q, n, s2, y)
-          : k_frsz1_decompress_vec<T, false, false><<<warps, 32, 0, s>>>(q, n, s2, y);
+      rnd ? launch(k_frsz1_decompress_vec<T, false, true>, warps, 32, 0, s, q, n, s2, y)
+          : launch(k_frsz1_decompress_vec<T, false, false>, warps, 32, 0, s, q, n, s2, y);
     return cuda_status(cudaGetLastError(), "legacy decompress launch");
   }
   const bool vec = reinterpret_cast<std::uintptr_t>(d_in) % 16 == 0;
   if (own)
-    k_frsz1_decompress<T, true><<<grid, kDecBlocks, 0, s>>>(q, n, eps * 2, y, vec);
+    launch(k_frsz1_decompress<T, true>, grid, kDecBlocks, 0, s, q, n, eps * 2, y, vec);
   else
-    k_frsz1_decompress<T, false><<<grid, kDecBlocks, 0, s>>>(q, n, eps * 2, y, vec);
+    launch(k_frsz1_decompress<T, false>, grid, kDecBlocks, 0, s, q, n, eps * 2, y, vec);
   return cuda_status(cudaGetLastError(), "legacy decompress launch");
 }
 
@@ -526,6 +529,7 @@ uint64_t frsz1_compressed_size(uint64_t n) { return n * sizeof(std::int16_t); }
 int frsz1_compress(int dtype, double epsilon, const void* d_values, uint64_t n, void* d_out, void* stream)
 {
   NvtxRange nvtx("frsz1_compress");
+  EarlyLaunch early;
   if (int rc = legacy_checks(dtype, epsilon, d_values, d_out, n)) return rc;
   const std::size_t es = dtype == FRSZ2_FLOAT ? 4 : 8;
   if (reinterpret_cast<std::uintptr_t>(d_values) % es != 0 || reinterpret_cast<std::uintptr_t>(d_out) % 2 != 0)
@@ -539,6 +543,7 @@ int frsz1_compress(int dtype, double epsilon, const void* d_values, uint64_t n, 
 int frsz1_decompress(int dtype, double epsilon, const void* d_in, uint64_t n, void* d_values, int flags, void* stream)
 {
   NvtxRange nvtx("frsz1_decompress");
+  EarlyLaunch early;
   if (int rc = legacy_checks(dtype, epsilon, d_in, d_values, n)) return rc;
   const std::size_t es = dtype == FRSZ2_FLOAT ? 4 : 8;
   if (reinterpret_cast<std::uintptr_t>(d_values) % es != 0 || reinterpret_cast<std::uintptr_t>(d_in) % 2 != 0)

@@ -36,6 +36,7 @@ constexpr int kBvThreads = 256;
 template<class T, int BITS>
 __global__ void __launch_bounds__(kBvThreads) k_compress_blockvec(Job j, std::uint64_t nb_full)
 {
+  enter_in_stream_order();
   static_assert(BITS <= 32, "codes of at most 32 bits");
   using Cfg = fast_cfg<T, BITS>;
   using U = typename Cfg::U;
@@ -138,7 +139,7 @@ cudaError_t launch_blockvec_one(const Job& j, std::uint64_t nb_full, cudaStream_
   if (nb_full == 0) return cudaSuccess;
   const std::uint64_t ctas = (nb_full + kBvThreads - 1) / kBvThreads;
   const unsigned grid = (unsigned)std::min<std::uint64_t>(ctas, (std::uint64_t)sm_count() * 32);
-  k_compress_blockvec<T, BITS><<<grid, kBvThreads, 0, s>>>(j, nb_full);
+  launch(k_compress_blockvec<T, BITS>, grid, kBvThreads, 0, s, j, nb_full);
   return cudaGetLastError();
 }
 

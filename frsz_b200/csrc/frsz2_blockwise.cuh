@@ -164,6 +164,7 @@ __device__ __forceinline__ void bw_commit(const std::uint8_t* g, std::uint8_t* s
 template<class T, int BITS>
 __global__ void __launch_bounds__(bw_threads<T>(), bw_min_ctas<T>()) k_compress_blockwise(Job j)
 {
+  enter_in_stream_order();
   using Cfg = fast_cfg<T, BITS>;
   using U = typename Cfg::U;
   using C = typename Cfg::C;
@@ -294,6 +295,7 @@ __global__ void __launch_bounds__(bw_threads<T>(), bw_min_ctas<T>()) k_compress_
 template<class T, int BITS>
 __global__ void __launch_bounds__(bw_threads<T>(), bw_min_ctas<T>()) k_decompress_blockwise(Job j)
 {
+  enter_in_stream_order();
   using Cfg = fast_cfg<T, BITS>;
   using U = typename Cfg::U;
   using C = typename Cfg::C;
@@ -425,9 +427,9 @@ cudaError_t launch_blockwise_one(bool compress, const Job& j, cudaStream_t s)
   const std::uint64_t ctas = (std::uint64_t)sm_count() * (std::uint64_t)per_sm;
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, std::min<std::uint64_t>((nb + nbc - 1) / nbc, ctas));
   if (compress)
-    k_compress_blockwise<T, BITS><<<grid, bw_threads<T>(), smem, s>>>(j);
+    launch(k_compress_blockwise<T, BITS>, grid, bw_threads<T>(), smem, s, j);
   else
-    k_decompress_blockwise<T, BITS><<<grid, bw_threads<T>(), smem, s>>>(j);
+    launch(k_decompress_blockwise<T, BITS>, grid, bw_threads<T>(), smem, s, j);
   return cudaGetLastError();
 }
 

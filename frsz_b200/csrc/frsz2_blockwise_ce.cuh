@@ -279,6 +279,7 @@ __device__ __forceinline__ void bwc_store_full(std::uint8_t* g, const std::uint8
 template<class T, int BITS, int E>
 __global__ void FRSZ2_BWC_BOUNDS_C(bw_threads<T>()) k_compress_bwc(Job j)
 {
+  enter_in_stream_order();
   using G = bwc_cfg<T, BITS, E, true>;
   using U = typename fp<T>::U;
   constexpr int NT = G::NT, W = G::W, BB = G::BB, NBC = G::NBC;
@@ -375,6 +376,7 @@ __global__ void FRSZ2_BWC_BOUNDS_C(bw_threads<T>()) k_compress_bwc(Job j)
 template<class T, int BITS, int E>
 __global__ void FRSZ2_BWC_BOUNDS_D(bw_threads<T>()) k_decompress_bwc(Job j)
 {
+  enter_in_stream_order();
   using G = bwc_cfg<T, BITS, E, false>;
   using U = typename fp<T>::U;
   using Cfg = fast_cfg<T, BITS>;
@@ -522,9 +524,9 @@ cudaError_t launch_bwc_one(bool compress, const Job& j, cudaStream_t s)
   const std::uint64_t nbc = compress ? (std::uint64_t)GC::NBC : (std::uint64_t)GD::NBC;
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, std::min<std::uint64_t>((nb + nbc - 1) / nbc, ctas));
   if (compress)
-    k_compress_bwc<T, BITS, E><<<grid, GC::NT, 0, s>>>(j);
+    launch(k_compress_bwc<T, BITS, E>, grid, GC::NT, 0, s, j);
   else
-    k_decompress_bwc<T, BITS, E><<<grid, GD::NT, 0, s>>>(j);
+    launch(k_decompress_bwc<T, BITS, E>, grid, GD::NT, 0, s, j);
   return cudaGetLastError();
 }
 

@@ -25,6 +25,12 @@ namespace {
 thread_local std::string g_last_error;
 }
 
+bool& early_launch()
+{
+  thread_local bool on = false;
+  return on;
+}
+
 int set_error(int code, const std::string& msg)
 {
   g_last_error = msg;
@@ -181,9 +187,9 @@ static int launch_compress_t(const Job& j, int dtype, cudaStream_t s, bool* used
   if (tile) {
     const unsigned grid = (unsigned)std::min<std::uint64_t>(j.tiles, 1u << 30);
     if (sizeof(T) == 8 && j.bits > 32)
-      k_compress_tile<T, std::uint64_t><<<grid, kNT, compress_smem<T>(j.bits), s>>>(j);
+      launch(k_compress_tile<T, std::uint64_t>, grid, kNT, compress_smem<T>(j.bits), s, j);
     else
-      k_compress_tile<T, std::uint32_t><<<grid, kNT, compress_smem<T>(j.bits), s>>>(j);
+      launch(k_compress_tile<T, std::uint32_t>, grid, kNT, compress_smem<T>(j.bits), s, j);
   } else if (blockwise_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_blockwise_f64(j.bits, true, j, s)
                                       : launch_blockwise_f32(j.bits, true, j, s),
@@ -193,14 +199,14 @@ static int launch_compress_t(const Job& j, int dtype, cudaStream_t s, bool* used
     const cudaError_t e = sizeof(T) == 8 ? launch_blockvec_f64(j.bits, j, full, s)
                                          : launch_blockvec_f32(j.bits, j, full, s);
     if (e != cudaSuccess) return cuda_status(e, "compress launch");
-    if (full * (std::uint64_t)j.E < j.n) k_compress_generic<T><<<1, kNT, 0, s>>>(job_from_block(j, full, sizeof(T)));
+    if (full * (std::uint64_t)j.E < j.n) launch(k_compress_generic<T>, 1, kNT, 0, s, job_from_block(j, full, sizeof(T)));
   } else if (chunked_ct_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_chunked_ct_f64(j.bits, true, j, s)
                                       : launch_chunked_ct_f32(j.bits, true, j, s),
                        "compress launch");
   } else {
     const std::uint64_t nb = (j.n + (std::uint64_t)j.E - 1) / (std::uint64_t)j.E;
-    k_compress_generic<T><<<grid_for(nb, kNT / 32), kNT, 0, s>>>(j);
+    launch(k_compress_generic<T>, grid_for(nb, kNT / 32), kNT, 0, s, j);
   }
   return cuda_status(cudaGetLastError(), "compress launch");
 }
@@ -219,9 +225,9 @@ static int launch_decompress_t(const Job& j, int dtype, cudaStream_t s, bool* us
   if (tile) {
     const unsigned grid = (unsigned)std::min<std::uint64_t>(j.tiles, 1u << 30);
     if (sizeof(T) == 8 && j.bits > 32)
-      k_decompress_tile<T, std::uint64_t><<<grid, kNT, decompress_smem<T>(j), s>>>(j);
+      launch(k_decompress_tile<T, std::uint64_t>, grid, kNT, decompress_smem<T>(j), s, j);
     else
-      k_decompress_tile<T, std::uint32_t><<<grid, kNT, decompress_smem<T>(j), s>>>(j);
+      launch(k_decompress_tile<T, std::uint32_t>, grid, kNT, decompress_smem<T>(j), s, j);
   } else if (blockwise_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_blockwise_f64(j.bits, false, j, s)
                                       : launch_blockwise_f32(j.bits, false, j, s),
@@ -232,7 +238,7 @@ static int launch_decompress_t(const Job& j, int dtype, cudaStream_t s, bool* us
                        "decompress launch");
   } else {
     const std::uint64_t nb = (j.n + (std::uint64_t)j.E - 1) / (std::uint64_t)j.E;
-    k_decompress_generic<T><<<grid_for(nb, kNT / 32), kNT, 0, s>>>(j);
+    launch(k_decompress_generic<T>, grid_for(nb, kNT / 32), kNT, 0, s, j);
   }
   return cuda_status(cudaGetLastError(), "decompress launch");
 }
@@ -255,11 +261,11 @@ static void launch_elements_t(const Job& j, const std::uint64_t* idx, std::uint6
   const unsigned grid = grid_for(count, kNT);
   const std::uint64_t mE = j.log2E < 0 ? ~0ull / (std::uint64_t)j.E + 1 : 0; // E not a power of two
   switch (j.W) {
-    case 8: k_decompress_elements<T, 8><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
-    case 16: k_decompress_elements<T, 16><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
-    case 32: k_decompress_elements<T, 32><<<grid, kNT, 0, s>>>(j, mE, idx, count, out); break;
+    case 8: launch(k_decompress_elements<T, 8>, grid, kNT, 0, s, j, mE, idx, count, out); break;
+    case 16: launch(k_decompress_elements<T, 16>, grid, kNT, 0, s, j, mE, idx, count, out); break;
+    case 32: launch(k_decompress_elements<T, 32>, grid, kNT, 0, s, j, mE, idx, count, out); break;
     default:
-      if constexpr (sizeof(T) == 8) k_decompress_elements<T, 64><<<grid, kNT, 0, s>>>(j, mE, idx, count, out);
+      if constexpr (sizeof(T) == 8) launch(k_decompress_elements<T, 64>, grid, kNT, 0, s, j, mE, idx, count, out);
   }
 }
 
@@ -637,6 +643,7 @@ int frsz2_compress(int dtype, int bits, int block_size, const void* d_values, ui
                    void* stream)
 {
   NvtxRange nvtx("frsz2_compress");
+  EarlyLaunch early;
   int rc = check_args(dtype, bits, block_size);
   if (rc) return rc;
   if (n == 0) return FRSZ2_OK;
@@ -651,6 +658,7 @@ int frsz2_decompress(int dtype, int bits, int block_size, const void* d_compress
                      void* stream)
 {
   NvtxRange nvtx("frsz2_decompress");
+  EarlyLaunch early;
   int rc = check_args(dtype, bits, block_size);
   if (rc) return rc;
   if (n == 0) return FRSZ2_OK;
@@ -691,6 +699,7 @@ int frsz2_compress_blocks(int dtype, int bits, int block_size, const void* d_val
                           uint64_t block_count, void* d_compressed, void* stream)
 {
   NvtxRange nvtx("frsz2_compress_blocks");
+  EarlyLaunch early;
   Layout L;
   if (int rc = block_range_args(dtype, bits, block_size, n, block_begin, block_count, d_values, d_compressed, &L))
     return rc;
@@ -706,6 +715,7 @@ int frsz2_decompress_blocks(int dtype, int bits, int block_size, const void* d_c
                             uint64_t block_begin, uint64_t block_count, void* d_values, void* stream)
 {
   NvtxRange nvtx("frsz2_decompress_blocks");
+  EarlyLaunch early;
   Layout L;
   if (int rc = block_range_args(dtype, bits, block_size, n, block_begin, block_count, d_values, d_compressed, &L))
     return rc;
@@ -721,6 +731,7 @@ int frsz2_decompress_elements(int dtype, int bits, int block_size, const void* d
                               const uint64_t* d_idx, uint64_t count, void* d_out, void* stream)
 {
   NvtxRange nvtx("frsz2_decompress_elements");
+  EarlyLaunch early;
   int rc = check_args(dtype, bits, block_size);
   if (rc) return rc;
   if (count == 0) return FRSZ2_OK;

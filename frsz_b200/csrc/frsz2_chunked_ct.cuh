@@ -45,6 +45,7 @@ constexpr int kChunkedUnroll = FRSZ2_CHUNKED_UNROLL;
 template<class T, int BITS>
 __global__ void __launch_bounds__(kNT) k_decompress_chunked_ct(Job j)
 {
+  enter_in_stream_order();
   using G = chunk_ct_cfg<T, BITS>;
   using Cfg = fast_cfg<T, BITS>;
   using U = typename Cfg::U;
@@ -230,6 +231,7 @@ __device__ __forceinline__ std::int64_t chunk_block_exponent(const typename fp<T
 template<class T, int BITS>
 __global__ void __launch_bounds__(kNT) k_compress_chunked_ct(Job j)
 {
+  enter_in_stream_order();
   using G = chunk_ct_cfg<T, BITS>;
   using Cfg = fast_cfg<T, BITS>;
   using U = typename Cfg::U;
@@ -357,9 +359,9 @@ cudaError_t launch_chunked_ct_one(bool compress, const Job& j, cudaStream_t s)
   const std::uint64_t ctas = (std::uint64_t)sm_count() * (std::uint64_t)per_sm;
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, std::min<std::uint64_t>((nb + nbc - 1) / nbc, ctas));
   if (compress)
-    k_compress_chunked_ct<T, BITS><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_chunked_ct<T, BITS>, grid, kNT, 0, s, j);
   else
-    k_decompress_chunked_ct<T, BITS><<<grid, kNT, 0, s>>>(j);
+    launch(k_decompress_chunked_ct<T, BITS>, grid, kNT, 0, s, j);
   return cudaGetLastError();
 }
 

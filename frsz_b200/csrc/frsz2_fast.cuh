@@ -973,6 +973,7 @@ template<class T, int BITS, int NT = kNT, int RPW = 2, bool PAD = false, int ESM
          bool GEN = false, bool HALF = false, bool WCR = false>
 __global__ void __launch_bounds__(NT, compress_ctas<T, BITS, PAD, ESM, MIS, GEN, HALF>()) k_compress_fast(Job j)
 {
+  enter_in_stream_order();
   __shared__ std::uint32_t s_rmax[2 * fast_cfg<T, BITS, NT, RPW>::ROWS];
   __shared__ __align__(16) std::uint32_t s_stage[stage_words<T, BITS, NT, RPW, ESM>::value];
   __shared__ std::uint32_t s_gmax[GEN ? (HALF ? 4 : 2) * fast_cfg<T, BITS, NT, RPW>::ROWS * 32 : 1];
@@ -1130,6 +1131,7 @@ template<class T, int BITS, int NT = kNT, int RPW = 2, bool PAD = false, int ESM
          bool GEN = false, bool HALF = false>
 __global__ void __launch_bounds__(NT) k_decompress_fast(Job j)
 {
+  enter_in_stream_order();
   const std::uint32_t mE = GEN ? 0xFFFFFFFFu / (std::uint32_t)j.E + 1u : 0u; // ceil(2^32 / E), E not a power of two
   for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
     fast_decompress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF>(j, tile, mE);
@@ -1140,6 +1142,7 @@ __global__ void __launch_bounds__(NT) k_decompress_fast(Job j)
 template<class T, int BITS, int NT, bool PAD>
 __global__ void __launch_bounds__(NT, 2048 / NT) k_decompress_fast_occ(Job j)
 {
+  enter_in_stream_order();
   for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
     fast_decompress_tile<T, BITS, NT, 2, PAD>(j, tile);
 }

@@ -41,14 +41,14 @@ cudaError_t launch_decompress_unaligned(const Job& j, cudaStream_t s, unsigned g
   const bool pad = job_padded(j);
   if constexpr ((SH & 1) != 0) {
     if (pad)
-      k_decompress_fast_occ<T, BITS, NT, true><<<grid, NT, 0, s>>>(t);
+      launch(k_decompress_fast_occ<T, BITS, NT, true>, grid, NT, 0, s, t);
     else
-      k_decompress_fast_occ<T, BITS, NT, false><<<grid, NT, 0, s>>>(t);
+      launch(k_decompress_fast_occ<T, BITS, NT, false>, grid, NT, 0, s, t);
   } else {
     if (pad)
-      k_decompress_fast<T, BITS, NT, 2, true><<<grid, NT, 0, s>>>(t);
+      launch(k_decompress_fast<T, BITS, NT, 2, true>, grid, NT, 0, s, t);
     else
-      k_decompress_fast<T, BITS, NT, 2, false><<<grid, NT, 0, s>>>(t);
+      launch(k_decompress_fast<T, BITS, NT, 2, false>, grid, NT, 0, s, t);
   }
   return cudaGetLastError();
 }
@@ -66,9 +66,9 @@ cudaError_t launch_fast_one(bool compress, const Job& j, cudaStream_t s, unsigne
     }
     if (job_padded(j)) {
       if (compress)
-        k_compress_fast<T, BITS, kNT, 2, true><<<grid, kNT, 0, s>>>(j);
+        launch(k_compress_fast<T, BITS, kNT, 2, true>, grid, kNT, 0, s, j);
       else
-        k_decompress_fast<T, BITS, kNT, 2, true><<<grid, kNT, 0, s>>>(j);
+        launch(k_decompress_fast<T, BITS, kNT, 2, true>, grid, kNT, 0, s, j);
       return cudaGetLastError();
     }
   }
@@ -76,13 +76,13 @@ cudaError_t launch_fast_one(bool compress, const Job& j, cudaStream_t s, unsigne
     // blocks of two warp rows (fp32 512, fp64 256 values): each warp's two rows
     // are consecutive, so a block's maximum needs no barrier (measured: fp64 12
     // bits 0.85 -> 1.01, fp32 8 bits 0.87 -> 1.03 of HBM; 32 / 64 bits even)
-    k_compress_fast<T, BITS, kNT, 2, false, 0, false, false, false, true><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_fast<T, BITS, kNT, 2, false, 0, false, false, false, true>, grid, kNT, 0, s, j);
     return cudaGetLastError();
   }
   if (compress)
-    k_compress_fast<T, BITS><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_fast<T, BITS>, grid, kNT, 0, s, j);
   else
-    k_decompress_fast<T, BITS><<<grid, kNT, 0, s>>>(j);
+    launch(k_decompress_fast<T, BITS>, grid, kNT, 0, s, j);
   return cudaGetLastError();
 }
 
@@ -122,9 +122,9 @@ cudaError_t launch_fast_gen_one(bool compress, const Job& j, cudaStream_t s, uns
     if (pad) return cudaErrorNotSupported;
     if (compress) {
       if (j.E <= 16 || j.E > 16 * fast_cfg<T, BITS>::P) return cudaErrorNotSupported;
-      k_compress_fast<T, BITS, kNT, 2, false, 0, false, true, true><<<grid, kNT, 0, s>>>(j);
+      launch(k_compress_fast<T, BITS, kNT, 2, false, 0, false, true, true>, grid, kNT, 0, s, j);
     } else {
-      k_decompress_fast<T, BITS, kNT, 2, false, 0, false, true, true><<<grid, kNT, 0, s>>>(j);
+      launch(k_decompress_fast<T, BITS, kNT, 2, false, 0, false, true, true>, grid, kNT, 0, s, j);
     }
     return cudaGetLastError();
   }
@@ -132,15 +132,15 @@ cudaError_t launch_fast_gen_one(bool compress, const Job& j, cudaStream_t s, uns
     // a lane reads its block's E / P lane maxima: up to 32 of them; padded
     // blocks keep the other kernels
     if (pad || j.E > 32 * fast_cfg<T, BITS>::P) return cudaErrorNotSupported;
-    k_compress_fast<T, BITS, kNT, 2, false, 0, false, true><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_fast<T, BITS, kNT, 2, false, 0, false, true>, grid, kNT, 0, s, j);
   } else if (pad) {
     // padded blocks: lanes place their bits by stream position (unaligned widths)
     if constexpr (fast_cfg<T, BITS>::ALIGNED)
       return cudaErrorNotSupported;
     else
-      k_decompress_fast<T, BITS, kNT, 2, true, 0, false, true><<<grid, kNT, 0, s>>>(j);
+      launch(k_decompress_fast<T, BITS, kNT, 2, true, 0, false, true>, grid, kNT, 0, s, j);
   } else {
-    k_decompress_fast<T, BITS, kNT, 2, false, 0, false, true><<<grid, kNT, 0, s>>>(j);
+    launch(k_decompress_fast<T, BITS, kNT, 2, false, 0, false, true>, grid, kNT, 0, s, j);
   }
   return cudaGetLastError();
 }
@@ -169,16 +169,16 @@ cudaError_t launch_fast_mis_one(bool compress, const Job& j, cudaStream_t s, uns
   if constexpr (!fast_cfg<T, BITS>::ALIGNED) {
     if (job_padded(j)) {
       if (compress)
-        k_compress_fast<T, BITS, kNT, 2, true, 0, true><<<grid, kNT, 0, s>>>(j);
+        launch(k_compress_fast<T, BITS, kNT, 2, true, 0, true>, grid, kNT, 0, s, j);
       else
-        k_decompress_fast<T, BITS, kNT, 2, true, 0, true><<<grid, kNT, 0, s>>>(j);
+        launch(k_decompress_fast<T, BITS, kNT, 2, true, 0, true>, grid, kNT, 0, s, j);
       return cudaGetLastError();
     }
   }
   if (compress)
-    k_compress_fast<T, BITS, kNT, 2, false, 0, true><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_fast<T, BITS, kNT, 2, false, 0, true>, grid, kNT, 0, s, j);
   else
-    k_decompress_fast<T, BITS, kNT, 2, false, 0, true><<<grid, kNT, 0, s>>>(j);
+    launch(k_decompress_fast<T, BITS, kNT, 2, false, 0, true>, grid, kNT, 0, s, j);
   return cudaGetLastError();
 }
 
@@ -205,9 +205,9 @@ template<class T, int BITS, int ESM>
 cudaError_t launch_small_one(bool compress, const Job& j, cudaStream_t s, unsigned grid)
 {
   if (compress)
-    k_compress_fast<T, BITS, kNT, 2, false, ESM><<<grid, kNT, 0, s>>>(j);
+    launch(k_compress_fast<T, BITS, kNT, 2, false, ESM>, grid, kNT, 0, s, j);
   else
-    k_decompress_fast<T, BITS, kNT, 2, false, ESM><<<grid, kNT, 0, s>>>(j);
+    launch(k_decompress_fast<T, BITS, kNT, 2, false, ESM>, grid, kNT, 0, s, j);
   return cudaGetLastError();
 }
 

@@ -313,9 +313,6 @@ __device__ __forceinline__ double warp_sums(double (&a)[N])
   }
 }
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 // Partial sums of the dot.  Unit u = slice * groups + group is JB vectors over
 // S positions, done by 2^lq warps of a CTA that take a part of the slice each;
 // a CTA's units are neighbouring groups of one slice, so its warps read w from
@@ -330,10 +327,10 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
   k_basis_dot(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ w, unsigned ns,
               unsigned groups, unsigned S, int lq, double* __restrict__ partials)
 {
+  enter_in_stream_order();
   static_assert((JB & (JB - 1)) == 0 && JB <= 8, "warp_sums");
   constexpr int Wb = fast_cfg<double, BITS>::W / 8;
   __shared__ double s_sum[kKW][JB];
-  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int warp = __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0);
   const unsigned unit = (blockIdx.x << (3 - lq)) + (unsigned)(warp >> lq);
@@ -442,10 +439,10 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
 __global__ void __launch_bounds__(kKT)
   k_basis_dot_final(const double* __restrict__ partials, unsigned int ns, double* __restrict__ h)
 {
+  enter_in_stream_order();
   __shared__ double s_red[kKW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const double* pj = partials + (std::uint64_t)blockIdx.x * ns;
-  pdl_wait(); // every partial sum is written
   double sum = 0.0;
   for (unsigned int b = tid; b < ns; b += kKT) sum += __ldcg(pj + b);
 #pragma unroll
@@ -467,6 +464,7 @@ __global__ void __launch_bounds__(kKT, axpy_ctas(BITS, NV))
   k_basis_axpy(const __grid_constant__ BasisParams bp, int m, BasisGeo g, const double* __restrict__ coef,
                double* __restrict__ y)
 {
+  enter_in_stream_order();
   constexpr int Wb = fast_cfg<double, BITS>::W / 8;
   __shared__ double s_c[kMaxBasis];
   for (int j = threadIdx.x; j < m; j += kKT) s_c[j] = __ldg(coef + j);
@@ -623,19 +621,10 @@ int launch_dot(const BasisParams& bp, int m, const BasisGeo& g, const double* w,
   DotPlan p;
   if (!dot_plan(m, g.n, NV, JB, &p)) return set_error(FRSZ2_EFAIL, "basis vectors too long");
   auto* rows = reinterpret_cast<double*>(static_cast<std::uint8_t*>(workspace) + 256);
-  k_basis_dot<BITS, NV, JB><<<p.grid, kKT, 0, s>>>(bp, m, g, w, p.ns, p.groups, p.S, p.lq, rows);
+  launch(k_basis_dot<BITS, NV, JB>, p.grid, kKT, 0, s, bp, m, g, w, p.ns, p.groups, p.S, p.lq, rows);
   if (int rc = cuda_status(cudaGetLastError(), "basis dot launch")) return rc;
-  // the sums' kernel is set up while the products run and waits for them
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)m);
-  cfg.blockDim = dim3(kKT);
-  cfg.stream = s;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
-  return cuda_status(cudaLaunchKernelEx(&cfg, k_basis_dot_final, (const double*)rows, p.ns, h), "basis dot launch");
+  launch(k_basis_dot_final, (unsigned)m, kKT, 0, s, rows, p.ns, h);
+  return cuda_status(cudaGetLastError(), "basis dot launch");
 }
 
 // The axpy's threads walk the vectors one after the other, so a short array has
@@ -650,9 +639,9 @@ int launch_axpy(const BasisParams& bp, int m, const BasisGeo& g, const double* c
   const std::uint64_t grid = (g.n + per - 1) / per;
   if (grid > 0x7FFFFFFFull) return set_error(FRSZ2_EFAIL, "basis vectors too long");
   if (four)
-    k_basis_axpy<BITS, 4, J4><<<(unsigned)grid, kKT, 0, s>>>(bp, m, g, coef, y);
+    launch(k_basis_axpy<BITS, 4, J4>, (unsigned)grid, kKT, 0, s, bp, m, g, coef, y);
   else
-    k_basis_axpy<BITS, NV, JN><<<(unsigned)grid, kKT, 0, s>>>(bp, m, g, coef, y);
+    launch(k_basis_axpy<BITS, NV, JN>, (unsigned)grid, kKT, 0, s, bp, m, g, coef, y);
   return cuda_status(cudaGetLastError(), "basis axpy launch");
 }
 
@@ -675,6 +664,7 @@ int frsz2_basis_dot(int dtype, int bits, int block_size, const void* const* basi
                     const void* w, void* h, void* workspace, uint64_t workspace_bytes, void* stream)
 {
   NvtxRange nvtx("frsz2_basis_dot");
+  EarlyLaunch early;
   BasisParams bp{};
   BasisGeo g{};
   if (int rc = basis_args(dtype, bits, block_size, basis, m, n, &bp, &g)) return rc;
@@ -704,6 +694,7 @@ int frsz2_basis_axpy(int dtype, int bits, int block_size, const void* const* bas
                      const void* coef, void* y, void* stream)
 {
   NvtxRange nvtx("frsz2_basis_axpy");
+  EarlyLaunch early;
   BasisParams bp{};
   BasisGeo g{};
   if (int rc = basis_args(dtype, bits, block_size, basis, m, n, &bp, &g)) return rc;
