@@ -1127,9 +1127,37 @@ __device__ __forceinline__ void fast_decompress_tile(const Job& j, std::uint64_t
   }
 }
 
+// The same budget for decompress: 0 for the plain instances (the unaligned widths
+// have their launch shapes), a cap where ptxas keeps too few CTAs of the others.
+// Measured like compress_ctas, no cap / 5 / 6 / 8 CTAs:
+//   blocks below a lane  fp32 E 2  8 bits 0.88 / 0.85 / 0.88 / 0.95, 16 bits 0.89 / 0.97
+//         / 0.99 / 1.00, 21 bits 1.06 / 1.05 / 1.04 / 0.94; E 4  8 bits 0.92 / 0.98 / 1.02 /
+//         1.01, 16 bits 1.05 / 1.05 / 1.04 / 1.04; fp64 E 2  13 bits 0.94 / 1.00 / 0.98 /
+//         1.02, 21 bits 1.05 / 1.05 / 1.04 / 1.03
+//   half lanes  fp32 E 20  6 bits 0.80 / 0.86 / 0.85 / 0.95, 24 bits 0.90 / 0.97 / 0.98 /
+//         1.02, 32 bits 1.07 / 1.01 / 1.04 / 1.01; fp64 no cap is best
+//   whole-block tiles, padded  fp32 E 24  13 bits 0.83 / 0.89 / 0.93 / 1.00, 21 bits 0.86 /
+//         0.90 / 0.97 / 0.97; fp64 E 24  13 bits 0.90 / 0.83 / 0.89 / 0.85, 21 bits 0.76 /
+//         0.83 / 0.85 / 0.93; unpadded  fp32 6 bits 0.98 / 0.89 / 0.95 / 1.01, 16 bits 1.03 /
+//         1.02 / 1.04 / 1.02; fp64 16 bits 1.02 / 0.95 / 1.02 / 0.99, 40 bits 1.01 / 1.03 /
+//         1.02 / 1.04
+//   values off by one  fp32 8 bits 0.82 / 0.85 / 0.82 / 0.63; fp64 8 bits 0.82 / 0.83 / 0.85
+//         / 0.59, 16 bits 0.90 / 0.86 / 0.92 / 0.66, 21 bits 0.74 / 0.73 / 0.70 / 0.74
+template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
+__host__ __device__ constexpr int decompress_ctas()
+{
+  constexpr bool F32 = sizeof(T) == 4;
+  if (ESM) return BITS <= (F32 && ESM == 4 ? 12 : 16) ? 8 : 0;
+  if (MIS) return PAD ? 0 : F32 ? (BITS <= 8 ? 5 : 0) : (BITS <= 16 ? 6 : 0);
+  if (HALF) return F32 && BITS <= 24 ? 8 : 0;
+  if (GEN && PAD) return F32 ? (BITS <= 16 ? 8 : 6) : (BITS > 16 && BITS <= 32 ? 8 : 0);
+  if (GEN) return F32 ? (BITS <= 7 ? 8 : 0) : (BITS > 32 && BITS <= 48 ? 8 : 0);
+  return 0;
+}
+
 template<class T, int BITS, int NT = kNT, int RPW = 2, bool PAD = false, int ESM = 0, bool MIS = false,
          bool GEN = false, bool HALF = false>
-__global__ void __launch_bounds__(NT) k_decompress_fast(Job j)
+__global__ void __launch_bounds__(NT, decompress_ctas<T, BITS, PAD, ESM, MIS, GEN, HALF>()) k_decompress_fast(Job j)
 {
   enter_in_stream_order();
   const std::uint32_t mE = GEN ? 0xFFFFFFFFu / (std::uint32_t)j.E + 1u : 0u; // ceil(2^32 / E), E not a power of two
