@@ -34,6 +34,7 @@ struct Class
   std::uint64_t tiles[kNumShapes] = { 0, 0, 0 };
   std::size_t desc_off[kNumShapes] = { 0, 0, 0 }; // first descriptor in the shape's array
   std::uint64_t tmap_off = 0;                     // first entry of the shape-0 tile index
+  bool padded = false;                            // some array's blocks end in pad bits
   batch_entry entry[kNumShapes] = {};
 };
 
@@ -117,7 +118,7 @@ int enqueue(frsz2_batch* p, bool compress, cudaStream_t s, int shape, int ctas_p
     cudaStream_t st = fork ? p->branch[ci % nb] : s;
     const cudaError_t e =
       per_tile && shape == 0 && c.entry[0].launch_tiles && p->d_tmap
-        ? c.entry[0].launch_tiles(compress, p->d_desc[0] + c.desc_off[0], p->d_tmap + c.tmap_off, tiles, st)
+        ? c.entry[0].launch_tiles(compress, c.padded, p->d_desc[0] + c.desc_off[0], p->d_tmap + c.tmap_off, tiles, st)
         : c.entry[shape].launch(compress, p->d_desc[shape] + c.desc_off[shape], (int)c.items.size(), tiles,
                                 (unsigned)grid, st);
     if (int rc = cuda_status(e, "batch launch")) return rc;
@@ -323,6 +324,7 @@ int frsz2_batch_create(const frsz2_batch_item* items, uint64_t count, frsz2_batc
       c = p->classes.end() - 1;
     }
     c->items.push_back((int)i);
+    c->padded |= job_padded(j);
   }
   for (int sh = 0; sh < kNumShapes; ++sh) {
     std::vector<BatchItem> desc;

@@ -18,8 +18,10 @@ struct BatchItem
   std::uint64_t tile_begin; // first tile of this array within its class
 };
 
+// fp64 at 21 bits in CTAs of 512 is held to four of them per SM, the count that
+// a plan of that width and shape can be configured to.
 template<class T, int BITS, int NT, int RPW, bool COMPRESS>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, sizeof(T) == 8 && BITS == 21 && NT == 512 && COMPRESS ? 4 : 0)
   k_batch_class(const BatchItem* __restrict__ items, int nitems, std::uint64_t total_tiles)
 {
   __shared__ std::uint32_t s_rmax[2 * (NT / 32) * RPW];
@@ -45,11 +47,25 @@ __global__ void __launch_bounds__(NT)
   }
 }
 
+// CTAs of 256 threads per SM that the per-tile compress kernel's registers must
+// allow.  It reads its array's descriptor before its values, so it needs more
+// tiles in flight than the single-array kernels: measured on B200, compress of
+// 1,024 arrays of 1 KiB to 64 MiB (8.6 GB moved), no cap 1,366 us, 6 CTAs 1,364, 8
+// at up to 16 bits 1,295, 8 at up to 32 bits 1,275; 2,000 arrays of up to 1 MiB 96.6 (6
+// CTAs), 92.4, 89.2 us.
+template<class T, int BITS>
+__host__ __device__ constexpr int batch_compress_ctas()
+{
+  return BITS <= 32 ? 8 : 0;
+}
+
 // One CTA per tile of a class's concatenated tile list, the tile's array
 // read from a per-tile index (one 4-byte load): the launch shape of the
 // single-array kernels, which hardware CTA scheduling balances across SMs.
-template<class T, int BITS, int NT, int RPW, bool COMPRESS>
-__global__ void __launch_bounds__(NT)
+// PADDED: some of the class's arrays have padded blocks (unaligned widths).  A
+// class without them takes the instance without their code.
+template<class T, int BITS, int NT, int RPW, bool COMPRESS, bool PADDED>
+__global__ void __launch_bounds__(NT, COMPRESS && !PADDED ? batch_compress_ctas<T, BITS>() : 0)
   k_batch_tiles(const BatchItem* __restrict__ items, const std::uint32_t* __restrict__ tile_item)
 {
   __shared__ std::uint32_t s_rmax[2 * (NT / 32) * RPW];
@@ -58,7 +74,7 @@ __global__ void __launch_bounds__(NT)
   const std::uint32_t it = __ldg(tile_item + t);
   const Job j = items[it].job;
   const std::uint64_t lt = t - items[it].tile_begin;
-  if constexpr (!fast_cfg<T, BITS, NT, RPW>::ALIGNED) {
+  if constexpr (PADDED) {
     if (job_padded(j)) {
       if (COMPRESS)
         fast_compress_tile<T, BITS, NT, RPW, true>(j, lt, s_rmax, s_stage, false);
@@ -73,17 +89,27 @@ __global__ void __launch_bounds__(NT)
     fast_decompress_tile<T, BITS, NT, RPW>(j, lt);
 }
 
-using batch_tiles_fn = cudaError_t (*)(bool compress, const BatchItem* items, const std::uint32_t* tile_item,
-                                       std::uint64_t tiles, cudaStream_t s);
+using batch_tiles_fn = cudaError_t (*)(bool compress, bool padded, const BatchItem* items,
+                                       const std::uint32_t* tile_item, std::uint64_t tiles, cudaStream_t s);
 
 template<class T, int BITS, int NT, int RPW>
-cudaError_t launch_batch_tiles(bool compress, const BatchItem* items, const std::uint32_t* tile_item,
+cudaError_t launch_batch_tiles(bool compress, bool padded, const BatchItem* items, const std::uint32_t* tile_item,
                                std::uint64_t tiles, cudaStream_t s)
 {
+  const unsigned grid = (unsigned)tiles;
+  if constexpr (!fast_cfg<T, BITS, NT, RPW>::ALIGNED) {
+    if (padded) {
+      if (compress)
+        k_batch_tiles<T, BITS, NT, RPW, true, true><<<grid, NT, 0, s>>>(items, tile_item);
+      else
+        k_batch_tiles<T, BITS, NT, RPW, false, true><<<grid, NT, 0, s>>>(items, tile_item);
+      return cudaGetLastError();
+    }
+  }
   if (compress)
-    k_batch_tiles<T, BITS, NT, RPW, true><<<(unsigned)tiles, NT, 0, s>>>(items, tile_item);
+    k_batch_tiles<T, BITS, NT, RPW, true, false><<<grid, NT, 0, s>>>(items, tile_item);
   else
-    k_batch_tiles<T, BITS, NT, RPW, false><<<(unsigned)tiles, NT, 0, s>>>(items, tile_item);
+    k_batch_tiles<T, BITS, NT, RPW, false, false><<<grid, NT, 0, s>>>(items, tile_item);
   return cudaGetLastError();
 }
 

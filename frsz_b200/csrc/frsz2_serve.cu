@@ -207,6 +207,7 @@ int launch_batch(frsz2_server* sv, Slot& s)
     if (is_fast[i]) ++per_key[key(s.reqs[i])];
   }
   std::uint64_t start[kKeys], fill[kKeys], tiles[kKeys] = {}, used = 0;
+  bool padded[kKeys] = {}; // some request's blocks end in pad bits
   for (int k = 0; k < kKeys; ++k) {
     start[k] = fill[k] = used;
     used += per_key[k];
@@ -220,6 +221,7 @@ int launch_batch(frsz2_server* sv, Slot& s)
     bi.job = job_of(q, out_ptr(q));
     bi.job.tiles = (q->r.n + (std::uint64_t)tv - 1) / (std::uint64_t)tv;
     bi.job.tile_blocks = (std::uint32_t)(tv / q->r.block_size);
+    padded[k] |= job_padded(bi.job);
     bi.tile_begin = tiles[k];
     tiles[k] += bi.job.tiles;
   }
@@ -278,7 +280,7 @@ int launch_batch(frsz2_server* sv, Slot& s)
     const int bits = rest - (is64 ? 65 : 0);
     const batch_entry e = is64 ? batch_class_f64(bits, 0) : batch_class_f32(bits, 0);
     cudaStream_t st = fork ? s.sub[ci++ % kSubStreams] : s.stream;
-    if (int rc = cuda_status(e.launch_tiles(comp, s.d_desc + start[k], s.d_tmap + tmap_start[k], tiles[k], st),
+    if (int rc = cuda_status(e.launch_tiles(comp, padded[k], s.d_desc + start[k], s.d_tmap + tmap_start[k], tiles[k], st),
                              "batch launch"))
       return rc;
   }
