@@ -500,6 +500,139 @@ __global__ void FRSZ2_BWC_BOUNDS_D(bw_threads<T>()) k_decompress_bwc(Job j)
   }
 }
 
+// ---------------------------------------------------------------- decompress by warps
+//
+// Arrays on 16-byte boundaries: a warp takes 32 blocks at a time, one per lane,
+// and goes on alone -- the lane reads its block's words straight from global
+// memory (neighbouring lanes' blocks are neighbours, so the sectors are shared
+// through L1), decodes, puts the values into the warp's own 32 * E values of shared
+// memory, and the warp stores them with 16-byte accesses.  Against the kernel
+// above, which stages images and values for the whole CTA, there is one pass
+// through shared memory instead of two and no barrier of the CTA (the
+// shared-memory queue and the barriers were its first stalls).
+//
+// Block bytes that are a multiple of 4 are read with the widest accesses they
+// allow; others as the aligned words around the block, moved by a funnel shift
+// (the array's last block, whose last word may reach past the buffer, byte by
+// byte).  One group of 32 blocks per warp where a group moves 1,200 bytes or more,
+// four below, where a CTA's own cost shows.  Measured on B200, 2^27 fp32 / 2^26 fp64
+// values, of the copy bandwidth, kernel above -> here (one group / four): fp64 21
+// bits E 5 0.84 -> 1.04 (1.04 / 0.98), 40 bits E 5 0.81 -> 1.06, 51 bits E 7 0.85 -> 1.05
+// (1.05 / 1.02), 21 bits E 3 0.93 -> 0.98 (0.94 / 0.98); fp32 32 bits E 5 0.98 -> 1.05 (1.05
+// / 1.02), 21 bits E 3 0.86 -> 0.92 (0.82 / 0.92), 6 bits E 5 0.83 -> 0.91 (0.74 / 0.91).
+template<class T, int BITS, int E>
+struct bww_cfg
+{
+  static constexpr int W = fast_cfg<T, BITS>::W;
+  static constexpr int BB = (E * BITS + W - 1) / W * (W / 8);
+  static constexpr int ROW = 32 * E * (int)sizeof(T);
+  static constexpr bool BIG = ROW + 32 * BB >= 1200;
+  // fp32 blocks of 3 or 5 values off word boundaries stay on the kernel above (16
+  // bits: E 3 0.85 there, 0.75 here; E 5 0.94 / 0.93; E 7 0.92 / 0.95)
+  static constexpr bool SERVES = BB % 4 == 0 || sizeof(T) == 8 || E > 5;
+  static constexpr int WARPS = BIG ? 8 : 4;
+  static constexpr int GROUPS = BIG ? 1 : 4; // groups of 32 blocks per warp
+  static constexpr bool WORDS = BB % 4 == 0; // blocks start on word boundaries
+  static constexpr int NW = (BB + 3) / 4;    // words of a block
+  static constexpr int NL = WORDS ? NW : (BB + (BB % 2 == 0 ? 2 : 3) + 3) / 4; // words around it
+};
+
+template<class T, int BITS, int E>
+__global__ void __launch_bounds__(32 * bww_cfg<T, BITS, E>::WARPS) k_decompress_bww(Job j)
+{
+  enter_in_stream_order();
+  using G = bww_cfg<T, BITS, E>;
+  using U = typename fp<T>::U;
+  using C = typename fast_cfg<T, BITS>::C;
+  constexpr int W = G::W, BB = G::BB, NW = G::NW, NL = G::NL;
+  constexpr int V = !G::WORDS ? 1 : BB % 16 == 0 ? 4 : BB % 8 == 0 ? 2 : 1;
+  using SWord = std::conditional_t<(W == 8), std::int8_t,
+                                   std::conditional_t<(W == 16), std::int16_t,
+                                                      std::conditional_t<(W == 32), std::int32_t, long long>>>;
+  __shared__ __align__(16) std::uint8_t s_row[G::WARPS][G::ROW];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const std::uint64_t nb = (j.n + E - 1) / E; // the last block may be partial
+  const std::uint64_t first = ((std::uint64_t)blockIdx.x * G::WARPS + warp) * (32 * G::GROUPS);
+  T* __restrict__ y = static_cast<T*>(j.values_out);
+  U* sv = reinterpret_cast<U*>(s_row[warp]) + lane * E;
+
+  std::uint32_t raw[NL + 1] = {};
+  int o = 0; // bits before the block in raw
+  SWord ex = 0;
+  auto load = [&](std::uint64_t b) {
+    if (b >= nb) return;
+    ex = __ldg(reinterpret_cast<const SWord*>(j.exps) + b);
+    const std::uint8_t* at = j.words + b * (std::uint64_t)BB;
+    if constexpr (!G::WORDS) {
+      if (b + 1 == nb) {
+        o = 0;
+#pragma unroll
+        for (int w = 0; w < NL; ++w) raw[w] = 0;
+#pragma unroll
+        for (int t = 0; t < BB; ++t) raw[t / 4] |= (std::uint32_t)__ldg(at + t) << (8 * (t % 4));
+        return;
+      }
+      const int low = (int)(reinterpret_cast<std::uintptr_t>(at) & 3u);
+      o = 8 * low;
+      at -= low;
+    }
+    const std::uint32_t* p = reinterpret_cast<const std::uint32_t*>(at);
+#pragma unroll
+    for (int w = 0; w < NL; w += V) {
+      if constexpr (V == 4) {
+        const uint4 t = __ldg(reinterpret_cast<const uint4*>(p + w));
+        raw[w] = t.x;
+        raw[w + 1] = t.y;
+        raw[w + 2] = t.z;
+        raw[w + 3] = t.w;
+      } else if constexpr (V == 2) {
+        const uint2 t = __ldg(reinterpret_cast<const uint2*>(p + w));
+        raw[w] = t.x;
+        raw[w + 1] = t.y;
+      } else {
+        // the last word only where the block reaches into it
+        if (G::WORDS || w + 1 < NL || o + 8 * BB > 32 * w) raw[w] = __ldg(p + w);
+      }
+    }
+  };
+  load(first + lane);
+#pragma unroll 1
+  for (int g = 0; g < G::GROUPS; ++g) {
+    const std::uint64_t b0 = first + 32 * (std::uint64_t)g;
+    if (b0 >= nb) return;
+    std::uint32_t seg[NW + 2];
+#pragma unroll
+    for (int w = 0; w < NW; ++w) seg[w] = G::WORDS ? raw[w] : __funnelshift_r(raw[w], raw[w + 1], o);
+    seg[NW] = seg[NW + 1] = 0;
+    C c[E];
+    unpack_all<0, BITS>(seg, c);
+    const std::int64_t e = ex;
+    if (g + 1 < G::GROUPS) load(b0 + 32 + lane); // in flight while this group is decoded
+    if (plain_exponent<T>(e)) {
+      const T inv = pow2<T>((int)e - BITS + 2);
+      const U zero_bits = sizeof(T) == 4 ? (U)((std::uint32_t)(e + 96) << 23) : (U)((std::uint64_t)(e + 992) << 52);
+#pragma unroll
+      for (int k = 0; k < E; ++k) sv[k] = decode_plain<T, BITS>(c[k], inv, zero_bits);
+    } else {
+#pragma unroll
+      for (int k = 0; k < E; ++k) sv[k] = to_bits<T>(from_code<T>((U)c[k], e, BITS));
+    }
+    __syncwarp();
+    const std::uint64_t v0 = b0 * E;
+    if (v0 + 32 * E <= j.n) {
+      uint4* dst = reinterpret_cast<uint4*>(y + v0);
+      const uint4* src = reinterpret_cast<const uint4*>(s_row[warp]);
+#pragma unroll
+      for (int q = 0; q < (G::ROW / 16 + 31) / 32; ++q)
+        if ((q + 1) * 32 <= G::ROW / 16 || q * 32 + lane < G::ROW / 16) __stcs(dst + q * 32 + lane, src[q * 32 + lane]);
+    } else {
+      const U* src = reinterpret_cast<const U*>(s_row[warp]);
+      for (int k = lane; k < 32 * E && v0 + k < j.n; k += 32) y[v0 + k] = from_bits<T>(src[k]);
+    }
+    __syncwarp(); // the row is free
+  }
+}
+
 // Launch of one (width, block size): a persistent grid of the resident CTAs,
 // fewer when there are fewer chunks.
 template<class T, int BITS, int E>
@@ -507,6 +640,16 @@ cudaError_t launch_bwc_one(bool compress, const Job& j, cudaStream_t s)
 {
   using GC = bwc_cfg<T, BITS, E, true>;
   using GD = bwc_cfg<T, BITS, E, false>;
+  using GW = bww_cfg<T, BITS, E>;
+  if constexpr (GW::SERVES) {
+    const std::uint64_t per = 32ull * GW::GROUPS * GW::WARPS;
+    const std::uint64_t ctas = ((j.n + (std::uint64_t)E - 1) / (std::uint64_t)E + per - 1) / per;
+    if (!compress && ctas <= 0x7FFFFFFFull &&
+        ((reinterpret_cast<std::uintptr_t>(j.values_out) | reinterpret_cast<std::uintptr_t>(j.words)) & 15u) == 0) {
+      launch(k_decompress_bww<T, BITS, E>, (unsigned)ctas, 32 * GW::WARPS, 0, s, j);
+      return cudaGetLastError();
+    }
+  }
   static std::atomic<int> resident[2];
   std::atomic<int>& slot = resident[compress ? 0 : 1];
   int per_sm = slot.load(std::memory_order_relaxed);
