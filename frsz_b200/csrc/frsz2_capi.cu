@@ -1,11 +1,11 @@
 // frsz2_capi.cu -- C ABI of libfrsz2_b200.so: argument checks, kernel choice,
 // launch geometry, and the host-buffer path with pipelined copies.
-#include "frsz2_blockvec.cuh"
 #include "frsz2_blockwise.cuh"
 #include "frsz2_chunked.cuh"
 #include "frsz2_chunked_ct.cuh"
 #include "frsz2_fast_dispatch.hpp"
 #include "frsz2_kernels.cuh"
+#include "frsz2_laneblock.cuh"
 #include "frsz2_launch.hpp"
 
 #include "../../include/frsz2_b200.h"
@@ -159,20 +159,6 @@ static cudaError_t try_fast(bool compress, const Job& j, cudaStream_t s)
 }
 
 
-// The blocks of a job from block b0 on (the generic kernel's share when the
-// blockvec kernel takes the whole blocks).
-static Job job_from_block(const Job& j, std::uint64_t b0, std::size_t es)
-{
-  Job t = j;
-  const std::uint64_t e0 = b0 * (std::uint64_t)j.E;
-  t.n = j.n - e0;
-  if (j.values_in) t.values_in = static_cast<const std::uint8_t*>(j.values_in) + e0 * es;
-  if (j.values_out) t.values_out = static_cast<std::uint8_t*>(j.values_out) + e0 * es;
-  t.exps = j.exps + b0 * (std::uint64_t)(j.W / 8);
-  t.words = j.words + b0 * (std::uint64_t)j.block_bytes;
-  return t;
-}
-
 template<class T>
 static int launch_compress_t(const Job& j, int dtype, cudaStream_t s, bool* used_tile)
 {
@@ -190,16 +176,14 @@ static int launch_compress_t(const Job& j, int dtype, cudaStream_t s, bool* used
       launch(k_compress_tile<T, std::uint64_t>, grid, kNT, compress_smem<T>(j.bits), s, j);
     else
       launch(k_compress_tile<T, std::uint32_t>, grid, kNT, compress_smem<T>(j.bits), s, j);
+  } else if (laneblock_eligible(j, sizeof(T), true, j.values_in, j.words)) {
+    return cuda_status(sizeof(T) == 8 ? launch_laneblock_f64(j.bits, true, j, s)
+                                      : launch_laneblock_f32(j.bits, true, j, s),
+                       "compress launch");
   } else if (blockwise_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_blockwise_f64(j.bits, true, j, s)
                                       : launch_blockwise_f32(j.bits, true, j, s),
                        "compress launch");
-  } else if (blockvec_eligible(j, sizeof(T), j.values_in, j.words)) {
-    const std::uint64_t full = j.n / (std::uint64_t)j.E;
-    const cudaError_t e = sizeof(T) == 8 ? launch_blockvec_f64(j.bits, j, full, s)
-                                         : launch_blockvec_f32(j.bits, j, full, s);
-    if (e != cudaSuccess) return cuda_status(e, "compress launch");
-    if (full * (std::uint64_t)j.E < j.n) launch(k_compress_generic<T>, 1, kNT, 0, s, job_from_block(j, full, sizeof(T)));
   } else if (chunked_ct_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_chunked_ct_f64(j.bits, true, j, s)
                                       : launch_chunked_ct_f32(j.bits, true, j, s),
@@ -228,6 +212,10 @@ static int launch_decompress_t(const Job& j, int dtype, cudaStream_t s, bool* us
       launch(k_decompress_tile<T, std::uint64_t>, grid, kNT, decompress_smem<T>(j), s, j);
     else
       launch(k_decompress_tile<T, std::uint32_t>, grid, kNT, decompress_smem<T>(j), s, j);
+  } else if (laneblock_eligible(j, sizeof(T), false, j.values_out, j.words)) {
+    return cuda_status(sizeof(T) == 8 ? launch_laneblock_f64(j.bits, false, j, s)
+                                      : launch_laneblock_f32(j.bits, false, j, s),
+                       "decompress launch");
   } else if (blockwise_eligible(j)) {
     return cuda_status(sizeof(T) == 8 ? launch_blockwise_f64(j.bits, false, j, s)
                                       : launch_blockwise_f32(j.bits, false, j, s),

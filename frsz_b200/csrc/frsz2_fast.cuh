@@ -635,7 +635,15 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
     bool any_special = false;
 #pragma unroll
     for (int rr = 0; rr < RPW; ++rr) {
-      const std::uint32_t m = raw_max<T, P, 0>(u[rr]);
+      std::uint32_t m;
+      if constexpr (GEN && sizeof(T) == 8 && BITS > 32 && !Cfg::ALIGNED) {
+        // the float maxima cost registers here (60 bits E 48 1.00 -> 0.91 of the time before)
+        m = K::raw(u[rr][0]);
+#pragma unroll
+        for (int i = 1; i < P; ++i) m = max(m, K::raw(u[rr][i]));
+      } else {
+        m = raw_max<T, P, 0>(u[rr]);
+      }
       km[rr] = m;
       any_special |= m >= K::SPECIAL;
     }
@@ -952,7 +960,8 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
 //   values off the 32-byte layout by one: fp32 16 bits 0.77 / 0.85 / 0.93 / 1.00,
 //         fp64 32 bits 0.88 / 0.88 / 0.94 / 1.02
 //   whole-block tiles (GEN): fp32 16 bits E 24 0.96 / 0.88 / 0.93 / 1.03, 32 bits
-//         E 24 0.91 / 1.00 / 1.05 / 1.03, E 20 0.62 / 0.84 / 0.90 / 0.90; fp64 16
+//         E 24 0.91 / 1.00 / 1.05 / 1.03, E 20 0.62 / 0.84 / 0.90 / 0.90 (27 bits E 96: 8 CTAs
+//         0.92 of the time without a cap's bandwidth); fp64 16
 //         bits E 48 0.92 / 0.82 / 0.91 / 0.96, 48 bits E 24 0.94 / 0.93 / 1.02 / 1.00
 //   blocks below a lane: fp32 16 bits E 2 0.88 / 0.94 / 0.94 / 0.92, E 4 24 bits
 //         1.03 / 1.05 / 1.04 / 1.04; fp64 16 bits E 2 0.98 / 1.00 / 1.03 / 0.99
@@ -963,6 +972,7 @@ __host__ __device__ constexpr int compress_ctas()
   if (PAD) return 0;
   if (HALF && half_keeps_integer_max<T, BITS>()) return 0;
   if (ESM) return F32 ? (BITS <= 16 ? 6 : ESM == 4 && BITS <= 24 ? 5 : 0) : (BITS > 8 && BITS <= 32 ? 6 : 0);
+  if (GEN && !fast_cfg<T, BITS>::ALIGNED) return BITS <= (F32 ? 20 : 32) ? 8 : 0;
   if (GEN) return BITS > 32 || (F32 && BITS == 32) ? 6 : 8;
   if (MIS) return 8;
   if (F32) return BITS <= 15 ? 8 : BITS == 16 ? 6 : BITS == 24 ? 5 : 0;
