@@ -134,8 +134,11 @@ static unsigned grid_for(std::uint64_t work_items, std::uint64_t per_cta)
 template<class T>
 static cudaError_t try_fast(bool compress, const Job& j, cudaStream_t s)
 {
+  // one CTA per tile, of down to half a tile each; an array beyond that (terabytes)
+  // goes to the kernels that loop
+  if (j.tiles > (1u << 29)) return cudaErrorNotSupported;
   const void* values = compress ? j.values_in : j.values_out;
-  const unsigned grid = (unsigned)std::min<std::uint64_t>(j.tiles, 1u << 30);
+  const unsigned grid = (unsigned)j.tiles;
   if (fast_eligible(j, sizeof(T) == 8, values, j.words))
     return sizeof(T) == 8 ? launch_fast_f64(j.bits, compress, j, s, grid)
                           : launch_fast_f32(j.bits, compress, j, s, grid);
@@ -151,7 +154,7 @@ static cudaError_t try_fast(bool compress, const Job& j, cudaStream_t s)
     const std::uint64_t tv = (std::uint64_t)tb * (std::uint64_t)j.E;
     t.tile_blocks = tb;
     t.tiles = (j.n + tv - 1) / tv;
-    const unsigned g = (unsigned)std::min<std::uint64_t>(t.tiles, 1u << 30);
+    const unsigned g = (unsigned)t.tiles;
     return sizeof(T) == 8 ? launch_fast_gen_f64(j.bits, compress, t, s, g)
                           : launch_fast_gen_f32(j.bits, compress, t, s, g);
   }

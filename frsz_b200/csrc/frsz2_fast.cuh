@@ -513,6 +513,59 @@ __device__ __forceinline__ void load_lane_exps(const std::uint8_t* p, std::int64
   }
 }
 
+// Whether a whole tile of compress is coded by an instance of its own, without the
+// partial tile's bounds: narrow widths, blocks below a lane, and values off the
+// 32-byte layout, where instructions bound the kernel.  Of the copy bandwidth, one
+// instance -> two, both without the loop (below): fp32 6 bits E 128 1.056 -> 1.078,
+// E 1024 0.92 -> 1.00, E 2 at 8 bits 0.80 -> 0.88, off by one 8 bits 0.98 -> 1.02; fp64 13 bits
+// E 512 1.03 -> 1.07, E 1 at 16 bits 0.99 -> 1.06.  Wider, the two cost registers (fp64
+// 33 bits 0.99 -> 0.84, off by one 51 bits 0.85 -> 0.79; fp32 padded 29 bits 0.95 -> 0.94;
+// whole-block tiles fp64 8 bits E 24 1.01 -> 0.95).
+template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
+__host__ __device__ constexpr bool compress_splits()
+{
+  constexpr bool F32 = sizeof(T) == 4;
+  if (GEN || HALF) return false;
+  if (MIS) return !PAD && (F32 ? BITS >= 8 && BITS <= 24 : BITS <= 32);
+  if (ESM) return BITS <= 16;
+  if (PAD) return !F32 && BITS <= 32;
+  return BITS <= (F32 ? 15 : 23);
+}
+
+// Whether a CTA takes its one tile (the grid is the tiles) or keeps a loop over
+// tiles that never comes round.  Without the loop's variables and branches there
+// are registers and instructions to spare: of the copy bandwidth, loop -> none,
+// compress fp32 6 bits E 128 0.94 -> 1.06, 9 bits E 64 0.99 -> 1.08, E 24 8 bits 0.94 ->
+// 1.03, off by one 12 bits 0.94 -> 1.02, padded 29 bits E 8 0.90 -> 0.95, fp64 9 bits E
+// 64 0.97 -> 1.08, 47 bits 0.98 -> 1.02; decompress fp32 off by one 16 bits 0.92 -> 1.03,
+// E 1 at 12 bits 0.75 -> 1.03, E 20 at 12 bits 0.91 -> 1.01, fp64 6 bits 0.91 -> 1.01,
+// padded 21 bits 0.93 -> 1.02.  The loop stays where more CTAs at once move less than
+// fewer (DRAM pages): compress fp32 16 bits 1.07 -> 1.06, 32 bits 1.065 -> 1.04, fp64 24
+// bits 1.09 -> 1.075; decompress fp32 13 bits 1.04 -> 1.00, fp64 29 bits 1.00 -> 0.97.
+// Every width was measured at E 32, most at E 256, fp32 2^27 / fp64 2^26 values.
+template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
+__host__ __device__ constexpr bool compress_straight()
+{
+  constexpr bool F32 = sizeof(T) == 4;
+  if (GEN || HALF || MIS || PAD) return true;
+  if (ESM) return BITS <= 16;
+  if (F32) return BITS <= 8 || (BITS <= 22 && BITS % 4 != 0);
+  return BITS <= 23 || (BITS > 32 && BITS % 2 == 1);
+}
+
+template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
+__host__ __device__ constexpr bool decompress_straight()
+{
+  constexpr bool F32 = sizeof(T) == 4;
+  if (MIS || HALF) return true;
+  if (GEN) return PAD || !(F32 ? BITS >= 8 && BITS <= 15 : BITS == 16); // fp32 12 bits E 24 1.03, 1.01 without
+  if (PAD) return !F32 || BITS <= 24;                                   // fp32 29 bits E 8 1.06, 1.05
+  if (ESM) return BITS <= (ESM == 4 ? 14 : 16) && (F32 || ESM == 1 || BITS > 8); // fp64 E 2 8 bits 1.01, 0.99
+  if (F32) return BITS <= 7 || BITS == 15 || (BITS >= 18 && BITS <= 23) || (BITS >= 25 && BITS <= 28) || BITS == 31;
+  return BITS <= 11 || (BITS >= 13 && BITS <= 15) || BITS == 19 || (BITS >= 21 && BITS <= 23) || BITS == 33 ||
+         BITS == 35 || BITS > 36;
+}
+
 // One tile of compress.  s_rmax: 2 * Cfg::ROWS words of shared memory (used
 // only when an exponent block spans several warp rows); s_stage:
 // stage_words<>::value words, 16-byte aligned.
@@ -527,8 +580,9 @@ __device__ __forceinline__ void load_lane_exps(const std::uint8_t* p, std::int64
 // WCR: blocks of exactly RPW warp rows (power-of-two E = RPW * 32 * P); a
 // warp's rows are consecutive (row = warp * RPW + rr), so a block lies in one
 // warp and its maximum needs no barrier.
+// FULL: the caller has seen that the tile is whole.
 template<class T, int BITS, int NT, int RPW_, bool PAD = false, int ESM = 0, bool MIS = false, bool GEN = false,
-         bool HALF = false, bool WCR = false>
+         bool HALF = false, bool WCR = false, bool FULL = false>
 __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t tile, std::uint32_t* s_rmax,
                                                    std::uint32_t* s_stage, bool more_tiles = true,
                                                    std::uint32_t* s_gmax = nullptr, std::uint32_t mE = 0)
@@ -550,7 +604,7 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
     const int TV = GEN ? TB * E : TE; // values of a whole tile
     const std::uint64_t e0 = tile * (std::uint64_t)TV;
     const std::uint64_t rem64 = j.n - e0;
-    const bool full = rem64 >= (std::uint64_t)TV;
+    const bool full = FULL || rem64 >= (std::uint64_t)TV;
     const int rem = full ? TV : (int)rem64;
     const int nbt = full ? TB : GEN ? (rem + E - 1) / E : ((rem + E - 1) >> log2E);
     const std::uint64_t b0 = tile * (std::uint64_t)TB;
@@ -637,7 +691,7 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
     for (int rr = 0; rr < RPW; ++rr) {
       std::uint32_t m;
       if constexpr (GEN && sizeof(T) == 8 && BITS > 32 && !Cfg::ALIGNED) {
-        // the float maxima cost registers here (60 bits E 48 1.00 -> 0.91 of the time before)
+        // the float maxima cost registers here (60 bits E 48: 0.91 of the integer maxima's speed)
         m = K::raw(u[rr][0]);
 #pragma unroll
         for (int i = 1; i < P; ++i) m = max(m, K::raw(u[rr][i]));
@@ -707,15 +761,18 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
         kc[rr] = warp_special ? __reduce_max_sync(0xFFFFFFFFu, kc[rr]) : km[rr];
       }
     } else if (G < 32) {
-      for (int s = 1; s < G; s <<= 1) {
+#pragma unroll
+      for (int s = 1; s < 32; s <<= 1) {
+        if (s >= G) break;
 #pragma unroll
         for (int rr = 0; rr < RPW; ++rr) km[rr] = max(km[rr], __shfl_xor_sync(0xFFFFFFFFu, km[rr], s));
-        if (warp_special) {
+      }
+      if (warp_special) {
+        for (int s = 1; s < G; s <<= 1) {
 #pragma unroll
           for (int rr = 0; rr < RPW; ++rr) kc[rr] = max(kc[rr], __shfl_xor_sync(0xFFFFFFFFu, kc[rr], s));
         }
-      }
-      if (!warp_special) {
+      } else {
 #pragma unroll
         for (int rr = 0; rr < RPW; ++rr) kc[rr] = km[rr];
       }
@@ -960,11 +1017,15 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
 //   values off the 32-byte layout by one: fp32 16 bits 0.77 / 0.85 / 0.93 / 1.00,
 //         fp64 32 bits 0.88 / 0.88 / 0.94 / 1.02
 //   whole-block tiles (GEN): fp32 16 bits E 24 0.96 / 0.88 / 0.93 / 1.03, 32 bits
-//         E 24 0.91 / 1.00 / 1.05 / 1.03, E 20 0.62 / 0.84 / 0.90 / 0.90 (27 bits E 96: 8 CTAs
-//         0.92 of the time without a cap's bandwidth); fp64 16
-//         bits E 48 0.92 / 0.82 / 0.91 / 0.96, 48 bits E 24 0.94 / 0.93 / 1.02 / 1.00
+//         E 24 0.91 / 1.00 / 1.05 / 1.03, E 20 0.62 / 0.84 / 0.90 / 0.90 (27 bits E 96
+//         runs at 0.92 of its uncapped speed with 8: unaligned widths above 20 bits
+//         have no cap); fp64 16 bits E 48 0.92 / 0.82 / 0.91 / 0.96, 48 bits E 24 0.94 /
+//         0.93 / 1.02 / 1.00
 //   blocks below a lane: fp32 16 bits E 2 0.88 / 0.94 / 0.94 / 0.92, E 4 24 bits
 //         1.03 / 1.05 / 1.04 / 1.04; fp64 16 bits E 2 0.98 / 1.00 / 1.03 / 0.99
+// These are of kernels with the loop over tiles; without it (compress_straight) the
+// caps rank the same, but for fp32 at 13 to 15 bits, 6 / 8 CTAs: 13 bits E 32 1.09 /
+// 1.06, E 1024 1.03 / 1.07, 14 bits E 32 1.08 / 1.06, 15 bits E 32 1.07 / 1.05.
 template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
 __host__ __device__ constexpr int compress_ctas()
 {
@@ -975,7 +1036,7 @@ __host__ __device__ constexpr int compress_ctas()
   if (GEN && !fast_cfg<T, BITS>::ALIGNED) return BITS <= (F32 ? 20 : 32) ? 8 : 0;
   if (GEN) return BITS > 32 || (F32 && BITS == 32) ? 6 : 8;
   if (MIS) return 8;
-  if (F32) return BITS <= 15 ? 8 : BITS == 16 ? 6 : BITS == 24 ? 5 : 0;
+  if (F32) return BITS <= 12 ? 8 : BITS <= 16 ? 6 : BITS == 24 ? 5 : 0;
   return BITS <= 30 && BITS != 24 ? 8 : 0;
 }
 
@@ -988,9 +1049,19 @@ __global__ void __launch_bounds__(NT, compress_ctas<T, BITS, PAD, ESM, MIS, GEN,
   __shared__ __align__(16) std::uint32_t s_stage[stage_words<T, BITS, NT, RPW, ESM>::value];
   __shared__ std::uint32_t s_gmax[GEN ? (HALF ? 4 : 2) * fast_cfg<T, BITS, NT, RPW>::ROWS * 32 : 1];
   const std::uint32_t mE = GEN ? 0xFFFFFFFFu / (std::uint32_t)j.E + 1u : 0u; // ceil(2^32 / E), E not a power of two
-  for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
-    fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR>(j, tile, s_rmax, s_stage,
-                                                                        tile + gridDim.x < j.tiles, s_gmax, mE);
+  if constexpr (compress_straight<T, BITS, PAD, ESM, MIS, GEN, HALF>()) {
+    const std::uint64_t tile = blockIdx.x;
+    constexpr std::uint64_t TE = fast_cfg<T, BITS, NT, RPW, ESM>::TE;
+    if (compress_splits<T, BITS, PAD, ESM, MIS, GEN, HALF>() && j.n - tile * TE >= TE)
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR, true>(j, tile, s_rmax, s_stage, false, s_gmax,
+                                                                              mE);
+    else
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR>(j, tile, s_rmax, s_stage, false, s_gmax, mE);
+  } else {
+    for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR>(j, tile, s_rmax, s_stage,
+                                                                          tile + gridDim.x < j.tiles, s_gmax, mE);
+  }
 }
 
 // ---------------------------------------------------------------- decompress
@@ -1171,8 +1242,12 @@ __global__ void __launch_bounds__(NT, decompress_ctas<T, BITS, PAD, ESM, MIS, GE
 {
   enter_in_stream_order();
   const std::uint32_t mE = GEN ? 0xFFFFFFFFu / (std::uint32_t)j.E + 1u : 0u; // ceil(2^32 / E), E not a power of two
-  for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
-    fast_decompress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF>(j, tile, mE);
+  if constexpr (decompress_straight<T, BITS, PAD, ESM, MIS, GEN, HALF>()) {
+    fast_decompress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF>(j, blockIdx.x, mE);
+  } else {
+    for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
+      fast_decompress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF>(j, tile, mE);
+  }
 }
 
 // The same with registers capped so that 2048 / NT CTAs fit on an SM (more
@@ -1181,8 +1256,12 @@ template<class T, int BITS, int NT, bool PAD>
 __global__ void __launch_bounds__(NT, 2048 / NT) k_decompress_fast_occ(Job j)
 {
   enter_in_stream_order();
-  for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
-    fast_decompress_tile<T, BITS, NT, 2, PAD>(j, tile);
+  if constexpr (decompress_straight<T, BITS, PAD, 0, false, false, false>()) {
+    fast_decompress_tile<T, BITS, NT, 2, PAD>(j, blockIdx.x);
+  } else {
+    for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
+      fast_decompress_tile<T, BITS, NT, 2, PAD>(j, tile);
+  }
 }
 
 // Whether a job's exponent blocks end in pad bits (E * bits not a multiple of

@@ -36,7 +36,7 @@ cudaError_t launch_decompress_unaligned(const Job& j, cudaStream_t s, unsigned g
     // tiles of NT / 32 * 2 rows (the caller checked E <= TE)
     t.tile_blocks = (std::uint32_t)(TE / j.E);
     t.tiles = (j.n + TE - 1) / TE;
-    grid = (unsigned)std::min<std::uint64_t>(t.tiles, 1u << 30);
+    grid = (unsigned)t.tiles;
   }
   const bool pad = job_padded(j);
   if constexpr ((SH & 1) != 0) {
