@@ -26,14 +26,15 @@
  * <= 65536.  Device pointers must be aligned to their element / word type.
  * Speed: power-of-two block sizes from 8 (fp32) / 4 (fp64) values up with a
  * 32-byte aligned buffer run at about the HBM bandwidth; values off the
- * 32-byte layout (a view such as x + 1) at 0.7-0.9 of it; block sizes 3, 5, 6,
- * 7 and 12 at 0.74-1.0, other block sizes up to 16 values at 0.4-0.8; block
+ * 32-byte layout (a view such as x + 1) at 0.8-1.05 of it; block sizes 3, 5, 6,
+ * 7 and 12 at 0.65-1.05, other block sizes up to 16 values at 0.4-0.9; block
  * sizes that are a multiple of 8 (fp32) / 4 (fp64) values without block
  * padding decompress at about the HBM bandwidth and compress at 0.75-1.0 (up
  * to 256 / 128 values), multiples of 4 / 2 decompress at about the HBM
- * bandwidth and compress at 0.55-0.7; other block sizes of 17-128 values decompress at
- * 0.33-0.89 and compress at 0.2-0.7; larger block sizes that are not powers of
- * two, or a buffer off the 32-byte layout, on slower general kernels.
+ * bandwidth and compress at 0.55-0.9; other block sizes of 17-128 values on a
+ * 16-byte aligned buffer decompress at 0.44-1.0 and compress at 0.25-0.97;
+ * larger block sizes that are not powers of two, or a buffer off the 32-byte
+ * layout, on slower general kernels.
  */
 #ifndef FRSZ2_B200_H
 #define FRSZ2_B200_H
@@ -89,10 +90,10 @@ int frsz2_decompress(int dtype, int bits, int block_size, const void* d_compress
 /* Host buffers: the same codec with the host<->device copies inside the call
  * (pinned memory recommended; pageable works).  Synchronous: returns when the
  * result is in host memory.  This is the drop-in for the reference's host-side
- * compress_cpu_impl / decompress_cpu_impl calls.  Ordinary memory goes through pinned slots
- * (up to 48 MiB pinned and 48 MiB of device memory per device, kept) by up to
- * 12 threads that end with the call, three quarters of the host's cores at
- * most; pinned buffers transfer directly. */
+ * compress_cpu_impl / decompress_cpu_impl calls.  Pinned buffers transfer
+ * directly.  Ordinary memory goes through pinned slots (up to 48 MiB pinned and
+ * 48 MiB of device memory per device, kept) by up to 12 threads that end with
+ * the call, three quarters of the host's cores at most. */
 int frsz2_compress_host(int dtype, int bits, int block_size, const void* h_values, uint64_t n, void* h_compressed,
                         void* stream);
 int frsz2_decompress_host(int dtype, int bits, int block_size, const void* h_compressed, uint64_t n, void* h_values,
