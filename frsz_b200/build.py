@@ -19,7 +19,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-shared"
 
 # translation units of the library (headers are tracked for staleness only);
 # compiled in parallel, then linked
-SOURCES = ["frsz2_capi.cu", "frsz2_fast_f32.cu", "frsz2_fast_f64.cu", "frsz2_fast_small_f32.cu",
+SOURCES = ["frsz2_capi.cu", "frsz2_host.cu", "frsz2_fast_f32.cu", "frsz2_fast_f64.cu", "frsz2_fast_small_f32.cu",
            "frsz2_fast_small_f64.cu", "frsz2_batch.cu", "frsz2_batch_f32.cu",
            "frsz2_batch_f64.cu", "frsz2_batch_static.cu", "frsz2_krylov.cu",
            "frsz2_serve.cu", "frsz1_legacy.cu", "frsz2_blockwise_f32.cu", "frsz2_blockwise_f64.cu",

@@ -2,7 +2,7 @@
 // translation units (argument checks, error state, kernel launchers).
 #pragma once
 
-#include "frsz2_kernels.cuh"
+#include "frsz2_job.hpp"
 
 #include <string>
 
@@ -22,6 +22,8 @@ int cuda_status(cudaError_t e, const char* what);
 int check_args(int dtype, int bits, int E);
 
 int sm_count();
+
+inline bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 
 // NVTX range around a C-ABI call (visible in nsys / ncu timelines; a no-op
 // without a tool attached).
@@ -45,5 +47,9 @@ Job job_for_slice(const Layout& L, int dtype, std::uint64_t b0, std::uint64_t nb
 // reports whether the tile kernel (rather than the generic one) was chosen.
 int launch_compress(const Job& j, int dtype, cudaStream_t s, bool* used_tile);
 int launch_decompress(const Job& j, int dtype, cudaStream_t s, bool* used_tile);
+
+// Enqueue the decode of the values at `count` indices.
+int launch_elements(const Job& j, int dtype, const std::uint64_t* idx, std::uint64_t count, void* out,
+                    cudaStream_t s);
 
 } // namespace frsz2b
