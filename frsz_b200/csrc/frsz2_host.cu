@@ -150,6 +150,9 @@ bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, co
   int workers = 0;
   while (workers < wanted && slot_init(S.slot[workers]) == FRSZ2_OK) ++workers;
   if (workers == 0) return false;
+  // the workers read the caller's input themselves, so what the caller's stream
+  // still holds (a copy into a pinned input, say) has to be done before they start
+  if ((*result = cuda_status(cudaEventSynchronize(S.ev_start), "event synchronize"))) return true;
 
   std::atomic<std::uint64_t> next{ 0 };
   std::atomic<int> status{ FRSZ2_OK };
@@ -200,7 +203,6 @@ bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, co
   };
   auto work = [&](int w) {
     int rc = w == 0 ? FRSZ2_OK : cuda_status(cudaSetDevice(dev), "cudaSetDevice");
-    if (!rc) rc = cuda_status(cudaStreamWaitEvent(S.slot[w].st, S.ev_start, 0), "stream wait");
     for (std::uint64_t k; !rc && status.load(std::memory_order_relaxed) == FRSZ2_OK &&
                           (k = next.fetch_add(1, std::memory_order_relaxed)) < slices;)
       rc = slice(S.slot[w], k);
