@@ -149,6 +149,9 @@ bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, co
     slices, (std::uint64_t)std::min<unsigned>(kHostWorkers, std::max(1u, hw ? hw - hw / 4 : 1u)));
   int workers = 0;
   while (workers < wanted && slot_init(S.slot[workers]) == FRSZ2_OK) ++workers;
+  // a slot that cannot be had leaves its error behind, which the next launch's
+  // check would take for its own
+  if (workers < wanted) cudaGetLastError();
   if (workers == 0) return false;
   // the workers read the caller's input themselves, so what the caller's stream
   // still holds (a copy into a pinned input, say) has to be done before they start

@@ -285,6 +285,12 @@ int main(int argc, char** argv)
     for (std::size_t n : sizes) both(n, true, true);
   } else if (s == "pending_pageable") { // a host function on the stream fills it
     for (std::size_t n : sizes) both(n, false, true);
+  } else if (s == "no_slots") { // no pinned memory to be had: the direct path
+    g_host_allocs = 0;
+    for (std::size_t n : sizes) both(n, false, true);
+  } else if (s == "some_slots") { // two workers' memory and half of a third's
+    g_host_allocs = 5;
+    for (std::size_t n : { sizes[4], sizes[0], sizes[4] }) both(n, false, true);
   } else {
     std::printf("unknown scenario\n");
     return 2;
