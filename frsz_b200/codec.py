@@ -62,9 +62,11 @@ def exponent_size(dtype, bits: int, block_size: int, n: int) -> int:
 
 def _size(code: int, bits: int, block_size: int, n: int) -> int:
     """compressed_size without a call into the library, for every launch's
-    check of its buffer; arguments out of range go to the library, which names
-    them."""
-    if not (4 <= bits <= (64 if code else 32) and 1 <= block_size <= 65536 and 0 <= n < 1 << 48):
+    check of its buffer.  Python integers only: those of numpy and torch would
+    wrap at their own width, so they go to the library, and so does what is out
+    of range, which it names."""
+    if not (type(bits) is type(block_size) is type(n) is int
+            and 4 <= bits <= (64 if code else 32) and 1 <= block_size <= 65536 and 0 <= n < 1 << 48):
         out = ctypes.c_uint64()
         check(lib().frsz2_compressed_size(code, bits, block_size, n, ctypes.byref(out)))
         return out.value
