@@ -52,7 +52,7 @@ class BatchPlan:
         self._h = h
 
     def _stream(self, stream):
-        return _stream_ptr(stream)
+        return _stream_ptr(stream or None)
 
     def compress(self, stream: Optional[torch.cuda.Stream] = None) -> None:
         check(lib().frsz2_batch_compress(self._h, self._stream(stream)))

@@ -23,7 +23,7 @@ class CompressedBasis:
         self.size = 0
 
     def _stream(self, stream):
-        return codec._stream_ptr(stream)
+        return codec._stream_ptr(stream or None)
 
     def set(self, j: int, v: torch.Tensor, stream=None) -> None:
         codec.compress(v.to(torch.float64).contiguous(), self.bits, self.block_size, out=self.buffers[j],

@@ -58,14 +58,14 @@ def compress_shard(values: torch.Tensor, n: int, bits: int, block_size: int, b0:
                    compressed: torch.Tensor, stream=None) -> None:
     """Compress blocks [b0, b1) of an n-value array; `values` holds exactly
     those blocks' values, `compressed` is the whole array's buffer."""
-    s = codec._stream_ptr(stream)
+    s = codec._stream_ptr(stream or None)
     check(lib().frsz2_compress_blocks(codec.dtype_code(values.dtype), bits, block_size, values.data_ptr(), n, b0,
                                       b1 - b0, compressed.data_ptr(), s))
 
 
 def decompress_shard(compressed: torch.Tensor, n: int, dtype, bits: int, block_size: int, b0: int, b1: int,
                      values: torch.Tensor, stream=None) -> None:
-    s = codec._stream_ptr(stream)
+    s = codec._stream_ptr(stream or None)
     check(lib().frsz2_decompress_blocks(codec.dtype_code(dtype), bits, block_size, compressed.data_ptr(), n, b0,
                                         b1 - b0, values.data_ptr(), s))
 
