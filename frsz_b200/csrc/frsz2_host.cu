@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdio>
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -160,7 +161,7 @@ bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, co
   std::atomic<std::uint64_t> next{ 0 };
   std::atomic<int> status{ FRSZ2_OK };
   std::mutex err_mu;
-  std::string err;
+  char err[256] = "";
   auto slice = [&](HostSlot& h, std::uint64_t k) -> int {
     const std::uint64_t b0 = k * per, nbk = std::min(per, L.nb - b0);
     const std::uint64_t e0 = b0 * (std::uint64_t)L.E;
@@ -204,16 +205,23 @@ bool host_codec_staged(Staging& S, bool compress, int dtype, const Layout& L, co
     }
     return FRSZ2_OK;
   };
-  auto work = [&](int w) {
-    int rc = w == 0 ? FRSZ2_OK : cuda_status(cudaSetDevice(dev), "cudaSetDevice");
-    for (std::uint64_t k; !rc && status.load(std::memory_order_relaxed) == FRSZ2_OK &&
-                          (k = next.fetch_add(1, std::memory_order_relaxed)) < slices;)
-      rc = slice(S.slot[w], k);
+  auto work = [&](int w) noexcept {
+    int rc = FRSZ2_OK;
+    bool thrown = false;
+    try {
+      rc = w == 0 ? FRSZ2_OK : cuda_status(cudaSetDevice(dev), "cudaSetDevice");
+      for (std::uint64_t k; !rc && status.load(std::memory_order_relaxed) == FRSZ2_OK &&
+                            (k = next.fetch_add(1, std::memory_order_relaxed)) < slices;)
+        rc = slice(S.slot[w], k);
+    } catch (...) { // a thread must not end the process, nor this one leave others behind
+      rc = FRSZ2_EFAIL;
+      thrown = true;
+    }
     if (rc) {
       cudaStreamSynchronize(S.slot[w].st); // nothing of this call stays in flight
       std::lock_guard<std::mutex> g(err_mu);
       if (status.load() == FRSZ2_OK) {
-        err = last_error(); // this thread's
+        std::snprintf(err, sizeof err, "%s", thrown ? "out of host memory" : last_error()); // this thread's
         status.store(rc);
       }
     }

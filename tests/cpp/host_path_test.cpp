@@ -291,6 +291,17 @@ int main(int argc, char** argv)
   } else if (s == "some_slots") { // two workers' memory and half of a third's
     g_host_allocs = 5;
     for (std::size_t n : { sizes[4], sizes[0], sizes[4] }) both(n, false, true);
+  } else if (s == "throwing") { // no memory on the host inside one worker or another
+    const auto x = values(sizes[4], 1);
+    std::vector<std::uint8_t> out(coded(x).size());
+    for (int k : { 0, 1, 5, 9 }) {
+      CUstream_st user;
+      g_throw_in = k;
+      CHECK(frsz2_compress_host(FRSZ2_DOUBLE, kBits, kE, x.data(), x.size(), out.data(), &user) == FRSZ2_EFAIL);
+      CHECK(std::strlen(frsz2b::last_error()) > 0);
+      g_throw_in = 1 << 30;
+      both(sizes[4], false, true); // the next call finds nothing of it in the way
+    }
   } else {
     std::printf("unknown scenario\n");
     return 2;

@@ -24,7 +24,8 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["plain", "pending_pinned", "pending_pageable", "no_slots", "some_slots"])
+@pytest.mark.parametrize("scenario", ["plain", "pending_pinned", "pending_pageable", "no_slots", "some_slots",
+                                      "throwing"])
 def test_scenario(program, scenario):
     r = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
