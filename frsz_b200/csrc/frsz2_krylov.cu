@@ -160,7 +160,12 @@ __device__ __forceinline__ void basis_codes(const std::uint32_t (&seg)[N], C (&c
 //   33 to 48 bits: the magnitude shifted up to 47 bits, or 2^15 when it is zero,
 //     at F = be + 1029 (a unit is 2^(be-46)).
 // Needs F to be a normal exponent field and be in the plain range:
-// be in [-959, 1002].
+// be in [-959, 1002].  A block of zeros (exponent field 0, be = -1023) decodes to
+// zeros; it comes with be = kZeroBlock, which gives the exponent field of be = 0
+// (F's bits above it shift out) and a base with the zero magnitude's low word, so
+// D - base is 0.
+constexpr int kZeroBlock = 1 << 16;
+
 template<int BITS>
 __device__ __forceinline__ bool direct_exponent(std::int64_t be)
 {
@@ -184,8 +189,9 @@ __device__ __forceinline__ void basis_values_direct(const basis_lane<BITS, NV>& 
   C c[NV];
   basis_codes<0, BITS>(seg, c);
   if constexpr (BITS <= 32) {
-    const int hi = (int)((std::uint32_t)(l.be + 1044) << 20);
-    const double base = __hiloint2double(hi, 0);
+    const std::uint32_t F = (std::uint32_t)(l.be + 1044);
+    const int hi = (int)(F << 20);
+    const double base = __hiloint2double(hi, (int)(F >> 16));
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const std::uint32_t t = c[k] << (32 - BITS);
@@ -194,8 +200,8 @@ __device__ __forceinline__ void basis_values_direct(const basis_lane<BITS, NV>& 
     }
   } else {
     static_assert(BITS <= 48, "magnitudes below 2^47");
-    const std::uint32_t hi = (std::uint32_t)(l.be + 1029) << 20;
-    const double base = __hiloint2double((int)hi, 0);
+    const std::uint32_t F = (std::uint32_t)(l.be + 1029), hi = F << 20;
+    const double base = __hiloint2double((int)hi, (int)(F >> 1 & 0x8000u));
 #pragma unroll
     for (int k = 0; k < NV; ++k) {
       const std::uint64_t t = c[k] << (48 - BITS); // sign at bit 47
@@ -239,10 +245,60 @@ __device__ __forceinline__ void basis_values_any(const basis_lane<BITS, NV>& l, 
 
 constexpr bool has_direct(int bits) { return bits <= 48; }
 
+// Bits of word i of a lane's stream that belong to magnitudes.
+template<int BITS, int NV>
+__host__ __device__ constexpr std::uint32_t magnitude_bits(int i)
+{
+  std::uint32_t m = 0;
+  for (int b = 32 * i; b < 32 * i + 32 && b < NV * BITS; ++b)
+    if (b % BITS != BITS - 1) m |= 1u << (b - 32 * i);
+  return m;
+}
+
+template<int BITS, int NV, int I = 0>
+__device__ __forceinline__ std::uint32_t any_magnitude(const basis_lane<BITS, NV>& l, int o)
+{
+  using L = basis_lane<BITS, NV>;
+  if constexpr (I == L::NW) {
+    return 0u;
+  } else {
+    std::uint32_t w;
+    if constexpr (L::ALIGNED)
+      w = l.w[I];
+    else
+      w = __funnelshift_r(l.w[I], l.w[I + 1], o);
+    constexpr std::uint32_t M = magnitude_bits<BITS, NV>(I);
+    return (w & M) | any_magnitude<BITS, NV, I + 1>(l, o);
+  }
+}
+
+// Makes the lanes of a step that holds exponents outside the direct range ready for
+// the direct arithmetic where they are blocks of zeros (the decoder gives +-0 for
+// zero magnitudes up to exponent -992).  False for the warp where any other such
+// lane is left; `other` has a bit for each vector of which it is this lane.
+// Sparse vectors: dot / axpy of 100 vectors of 2^22 values with half of their blocks
+// zero, us, through the decoder's arithmetic -> here: 16 bits 900 / 825 -> 209 / 191,
+// 21 bits 1,075 / 885 -> 318 / 282, 32 bits 969 / 872 -> 272 / 264, 48 bits 1,113 / 1,028
+// -> 500 / 467; 1 % zero, 16 bits 342 / 335 -> 185 / 170.
+template<int BITS, int NV, int JB>
+__device__ __forceinline__ bool settle_zeros(basis_lane<BITS, NV> (&l)[JB], int o, unsigned& other)
+{
+  other = 0;
+#pragma unroll
+  for (int jj = 0; jj < JB; ++jj)
+    if (!direct_exponent<BITS>(l[jj].be)) {
+      if (l[jj].be <= -992 && any_magnitude<BITS, NV>(l[jj], o) == 0)
+        l[jj].be = kZeroBlock;
+      else
+        other |= 1u << jj;
+    }
+  return !__any_sync(0xFFFFFFFFu, other != 0);
+}
+
 // acc + sum of v[k] * w[k], k < cnt, in order: a lane of a step that holds an
-// exponent outside the direct range (loads again, off the fast path).  JB gives
-// each kernel its own copy: nvcc 12.9 fails on one that is shared by kernels of
-// different register bounds.
+// exponent outside the direct range which is no block of zeros (loads again, off
+// the fast path; eight values per lane).  JB gives each kernel its own copy: nvcc
+// 12.9 fails on one that is shared by kernels of different register bounds.
 template<int BITS, int NV, int JB>
 __device__ __noinline__ double slow_lane_dot(const std::uint8_t* exp, const std::uint8_t* words, std::uint64_t S,
                                              const double* w, int cnt, double acc)
@@ -268,6 +324,135 @@ __device__ __noinline__ void slow_lane_axpy(const std::uint8_t* exp, const std::
   basis_values_any<BITS, NV>(l, (int)(S & 31u), v);
 #pragma unroll
   for (int k = 0; k < NV; ++k) y[k] = fma(c, v[k], y[k]);
+}
+
+// A lane's values of w: 32-byte loads where `whole` says that w is aligned and all
+// of them are there, else those below cnt one by one.
+template<int NV>
+__device__ __forceinline__ void load_w(const double* w, bool whole, int cnt, double (&wv)[NV])
+{
+  if (whole) {
+#pragma unroll
+    for (int h = 0; h < NV; h += 4) {
+      std::uint32_t t[8];
+      asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                   : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+                   : "l"(w + h));
+#pragma unroll
+      for (int k = 0; k < 4; ++k) wv[h + k] = __hiloint2double((int)t[2 * k + 1], (int)t[2 * k]);
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) wv[k] = k < cnt ? __ldg(w + k) : 0.0;
+  }
+}
+
+// What is left of a warp's part of a slice (positions from p on) once a step holds
+// an exponent outside the direct range, as vectors with blocks of zeros do; the
+// kernels of four values per lane leave it to this.  Out of line, so that the loop of
+// the other steps keeps its registers: in line, as the kernels of eight values have
+// it, dense vectors lose there (dot of 100 vectors of 2^22 at 48 bits 391 -> 404 us;
+// axpy of 30 of 300,007 at 16 bits 6.8 -> 8.2, at 21 bits 9.3 -> 10.5), and out of
+// line with eight those do (dot at 32 bits 258 -> 272 us, axpy at 21 bits 233 -> 252).
+template<int BITS, int NV, int JB>
+__device__ __noinline__ void rest_of_dot(const std::uint8_t* const* bufs, int nv, std::uint64_t exp_bytes, int log2E,
+                                         const double* w, std::uint64_t pos0, int p, int len, double* sums)
+{
+  constexpr int Wb = fast_cfg<double, BITS>::W / 8;
+  const int lane = threadIdx.x & 31;
+  const bool wvec = (reinterpret_cast<std::uintptr_t>(w) & 31u) == 0;
+  double acc[JB];
+#pragma unroll
+  for (int jj = 0; jj < JB; ++jj) acc[jj] = sums[jj];
+#pragma unroll 1
+  for (; p - lane * NV < len; p += 32 * NV) {
+    const std::uint64_t idx = pos0 + (std::uint64_t)p;
+    const std::uint64_t S0 = idx * (std::uint64_t)BITS;
+    const std::uint64_t eo = (idx >> log2E) * Wb;
+    const int o = (int)(S0 & 31u);
+    basis_lane<BITS, NV> l[JB];
+#pragma unroll
+    for (int jj = 0; jj < JB; ++jj) {
+      l[jj].be = 0;
+      if (p < len && jj < nv) basis_load<BITS, NV>(bufs[jj] + eo, bufs[jj] + exp_bytes, S0, l[jj]);
+    }
+    double wv[NV];
+    load_w<NV>(w + idx, wvec && p + NV <= len, len - p, wv);
+    unsigned other;
+    if (settle_zeros<BITS, NV, JB>(l, o, other)) {
+#pragma unroll
+      for (int jj = 0; jj < JB; ++jj) {
+        double v[NV];
+        basis_values_direct<BITS, NV>(l[jj], o, v);
+        double t = v[0] * wv[0];
+#pragma unroll
+        for (int k = 1; k < NV; ++k) t = fma(v[k], wv[k], t);
+        acc[jj] += t;
+      }
+    } else if (p < len) {
+#pragma unroll
+      for (int jj = 0; jj < JB; ++jj) {
+        double v[NV];
+        if ((other >> jj & 1u) == 0)
+          basis_values_direct<BITS, NV>(l[jj], o, v);
+        else
+          basis_values_any<BITS, NV>(l[jj], o, v);
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < NV; ++k)
+          if (p + k < len) t = fma(v[k], wv[k], t);
+        acc[jj] += t;
+      }
+    }
+    __syncwarp();
+  }
+#pragma unroll
+  for (int jj = 0; jj < JB; ++jj) sums[jj] = acc[jj];
+}
+
+// The same for the axpy: the vectors from the step's first on.
+template<int BITS, int NV, int JB>
+__device__ __noinline__ void rest_of_axpy(const std::uint8_t* const* bufs, int left, std::uint64_t exp_bytes,
+                                          std::uint64_t eo, std::uint64_t S0, bool in, const double* coef, double* y)
+{
+  const int o = (int)(S0 & 31u);
+  double acc[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) acc[k] = y[k];
+#pragma unroll 1
+  for (; left > 0; left -= JB, bufs += JB, coef += JB) {
+    basis_lane<BITS, NV> l[JB];
+#pragma unroll
+    for (int jj = 0; jj < JB; ++jj) {
+      l[jj].be = 0;
+      if (in && jj < left) basis_load<BITS, NV>(bufs[jj] + eo, bufs[jj] + exp_bytes, S0, l[jj]);
+    }
+    unsigned other;
+    const bool direct = settle_zeros<BITS, NV, JB>(l, o, other);
+    auto add = [&](auto value) {
+#pragma unroll
+      for (int jj = 0; jj < JB; ++jj)
+        if (jj < left) {
+          double v[NV];
+          value(jj, v);
+          const double cj = coef[jj];
+#pragma unroll
+          for (int k = 0; k < NV; ++k) acc[k] = fma(cj, v[k], acc[k]);
+        }
+    };
+    if (direct)
+      add([&](int jj, double (&v)[NV]) { basis_values_direct<BITS, NV>(l[jj], o, v); });
+    else
+      add([&](int jj, double (&v)[NV]) {
+        if ((other >> jj & 1u) == 0)
+          basis_values_direct<BITS, NV>(l[jj], o, v);
+        else
+          basis_values_any<BITS, NV>(l[jj], o, v);
+      });
+    __syncwarp();
+  }
+#pragma unroll
+  for (int k = 0; k < NV; ++k) y[k] = acc[k];
 }
 
 // Sums of N (a power of two up to 32) values over the warp in a fixed order:
@@ -346,7 +531,9 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
     double acc[JB];
 #pragma unroll
     for (int jj = 0; jj < JB; ++jj) acc[jj] = 0.0;
-    for (int p = lane * NV; p - lane * NV < len; p += 32 * NV) {
+    int p = lane * NV;
+    bool rest = false;
+    for (; p - lane * NV < len; p += 32 * NV) {
       const bool in = p < len;
       const std::uint64_t idx = pos0 + (std::uint64_t)p;
       const std::uint64_t S0 = idx * (std::uint64_t)BITS;
@@ -364,27 +551,21 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
         }
       }
       double wv[NV];
-      if (in && wvec && p + NV <= len) {
-#pragma unroll
-        for (int h = 0; h < NV; h += 4) {
-          std::uint32_t t[8];
-          asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                       : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]),
-                         "=r"(t[7])
-                       : "l"(w + idx + h));
-#pragma unroll
-          for (int k = 0; k < 4; ++k) wv[h + k] = __hiloint2double((int)t[2 * k + 1], (int)t[2 * k]);
-        }
-      } else {
-#pragma unroll
-        for (int k = 0; k < NV; ++k) wv[k] = p + k < len ? __ldg(w + idx + k) : 0.0;
-      }
+      load_w<NV>(w + idx, wvec && p + NV <= len, len - p, wv);
       const int o = (int)(S0 & 31u);
-      bool slow = false;
       if constexpr (has_direct(BITS)) {
+        bool slow = false;
 #pragma unroll
         for (int jj = 0; jj < JB; ++jj) slow |= !direct_exponent<BITS>(l[jj].be);
-        if (!__any_sync(0xFFFFFFFFu, slow)) {
+        slow = __any_sync(0xFFFFFFFFu, slow);
+        if constexpr (NV == 4) {
+          rest = slow;
+          if (rest) break;
+        } else if (slow) {
+          unsigned other;
+          slow = !settle_zeros<BITS, NV, JB>(l, o, other);
+        }
+        if (NV == 4 || !slow) {
 #pragma unroll
           for (int jj = 0; jj < JB; ++jj) {
             double v[NV];
@@ -414,6 +595,16 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
             if (p + k < len) t = fma(v[k], wv[k], t);
           acc[jj] += t;
         }
+      }
+    }
+    if constexpr (has_direct(BITS) && NV == 4) {
+      if (rest) {
+        double t[JB];
+#pragma unroll
+        for (int jj = 0; jj < JB; ++jj) t[jj] = acc[jj];
+        rest_of_dot<BITS, NV, JB>(bp.buf + j0, nv, g.exp_bytes, g.log2E, w, pos0, p, len, t);
+#pragma unroll
+        for (int jj = 0; jj < JB; ++jj) acc[jj] = t[jj];
       }
     }
     sum = warp_sums<JB>(acc);
@@ -502,6 +693,10 @@ __global__ void __launch_bounds__(kKT, axpy_ctas(BITS, NV))
 #pragma unroll
       for (int jj = 0; jj < JB; ++jj) slow |= !direct_exponent<BITS>(l[jj].be);
       slow = __any_sync(0xFFFFFFFFu, slow);
+      if (NV == 8 && slow) {
+        unsigned other;
+        slow = !settle_zeros<BITS, NV, JB>(l, o, other);
+      }
     }
     if (!slow) {
 #pragma unroll
@@ -516,17 +711,21 @@ __global__ void __launch_bounds__(kKT, axpy_ctas(BITS, NV))
 #pragma unroll
           for (int k = 0; k < NV; ++k) acc[k] = fma(cj, v[k], acc[k]);
         }
-    } else {
-      if (in) {
-        double t[NV];
+    } else if constexpr (has_direct(BITS)) {
+      double t[NV];
 #pragma unroll
-        for (int k = 0; k < NV; ++k) t[k] = acc[k];
+      for (int k = 0; k < NV; ++k) t[k] = acc[k];
+      if constexpr (NV == 4)
+        rest_of_axpy<BITS, NV, JB>(bp.buf + j0, m - j0, g.exp_bytes, eo, S0, in, s_c + j0, t);
+      else if (in)
         for (int j = j0; j < min(m, j0 + JB); ++j)
           slow_lane_axpy<BITS, NV>(bp.buf[j] + eo, bp.buf[j] + g.exp_bytes, S0, s_c[j], t);
 #pragma unroll
-        for (int k = 0; k < NV; ++k) acc[k] = t[k];
-      }
-      __syncwarp();
+      for (int k = 0; k < NV; ++k) acc[k] = t[k];
+      if constexpr (NV == 4)
+        break;
+      else
+        __syncwarp();
     }
   }
   if (whole) {
