@@ -104,22 +104,32 @@ __device__ __forceinline__ T legacy_sub(T a, T b)
 // 0.5, so |p| + (2^51 + 0.5) rounded toward zero holds floor(2 |p| + 1) in its
 // low word, and dropping the last bit leaves floor(|p| + 0.5) (the exact sum
 // is truncated once, so |p| = 0.5 - 2^-54 gives 0 as std::round does).
-// `off` collects the bits that show a value outside that range: the sum's
-// high word differs from 2^51's (|p| >= 2^30, Inf, NaN), or its low word
-// reaches 2^25.
 template<class T>
-__device__ __forceinline__ int legacy_quantize_int(T x, double inv, std::uint32_t& off_hi, std::uint32_t& off_lo)
+__device__ __forceinline__ int legacy_quantize_int(T x, double inv)
 {
   const double r = __dadd_rz(fabs(__dmul_rn((double)x, inv)), 2251799813685248.5); // 2^51 + 0.5
   const std::uint32_t lo = (std::uint32_t)__double2loint(r);
-  off_hi |= (std::uint32_t)__double2hiint(r) ^ 0x43200000u;
-  off_lo |= lo;
   int sx;
   if constexpr (sizeof(T) == 4)
     sx = __float_as_int(x) >> 31;
   else
     sx = __double2hiint(x) >> 31;
   return ((int)(lo >> 1) ^ sx) - sx; // inv > 0: p has x's sign
+}
+
+// Whether every p of N values is below 2^24 (false with a NaN or an infinity):
+// from the largest magnitude, fp64's by its high word (three-input float maxima,
+// see raw_max), rounded up.
+template<class T, int N>
+__device__ __forceinline__ bool legacy_in_range(const T (&x)[N], double inv)
+{
+  typename fp<T>::U u[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) u[k] = to_bits<T>(x[k]);
+  const std::uint32_t m = raw_max<T, N, 0>(u);
+  if (m >= key_of<T>::SPECIAL) return false;
+  const double most = sizeof(T) == 4 ? (double)__uint_as_float(m) : __hiloint2double((int)m, -1);
+  return __dmul_rn(most, inv) < 16777216.0;
 }
 
 // Two differences as saturated int16 in one word (lo in the low half).
@@ -132,25 +142,31 @@ __device__ __forceinline__ std::uint32_t pack_sat_s16(int lo, int hi)
 
 constexpr int kComV = 8; // values per thread: a warp's 32 threads take one block of 256
 
-// A warp codes one block of 256 values, 8 consecutive ones per thread, so the
-// first thread's predecessor is the block's start and the others' is one
-// shuffle away.  Whole blocks on aligned pointers quantize to integers
-// (legacy_quantize_int) and saturate two differences per instruction; a warp
-// that meets a value outside its range codes its block with the float
-// arithmetic.  Bound by DRAM (before, by the instructions of the float
-// arithmetic: 28 per value, 16 now); measured on B200, 2^26 values: fp32 76.1 ->
-// 62.9 us (0.81 -> 0.98 of the copy bandwidth), fp64 111 -> 95.7 us.
-template<class T>
+// A warp codes one block of 256 values, 8 per thread.  VEC, aligned pointers: 8
+// consecutive ones, so the first thread's predecessor is the block's start and the
+// others' is one shuffle away.  Otherwise value k of a thread is the warp's
+// 32 k + lane, so that loads and stores of single values are coalesced.  Values
+// quantize to integers (legacy_quantize_int) and VEC saturates two differences per
+// instruction; a warp that meets a value outside the range codes its block with
+// the float arithmetic.  VEC is bound by DRAM (before, by the instructions of the
+// float arithmetic: 28 per value, 16 now); measured on B200, 2^26 values,
+// float arithmetic only -> here: fp32 78 -> 57.7 us (1.06 of the copy bandwidth), fp64
+// 113 -> 95 us; off alignment fp32 127 -> 65.3 us, fp64 115 -> 94.6 us (8 consecutive
+// values per thread there: 103 and 163 us); every value out of the range, fp32 78 ->
+// 68.8 us.
+template<class T, bool VEC>
 __global__ void __launch_bounds__(256) k_frsz1_compress(const T* __restrict__ x, std::uint64_t n, double inv,
-                                                        std::int16_t* __restrict__ out, bool vec)
+                                                        std::int16_t* __restrict__ out)
 {
   enter_in_stream_order();
   static_assert(kComV * 32 == kLegacyBlock, "one block per warp");
   constexpr int V = kComV;
   const int lane = threadIdx.x & 31;
-  const std::uint64_t i0 = ((std::uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * V;
+  const std::uint64_t w0 = ((std::uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u)) * V; // the warp's block
+  const std::uint64_t i0 = VEC ? w0 + lane * V : w0 + lane; // the thread's first value
+  constexpr int STEP = VEC ? 1 : 32;
   T xv[V];
-  const bool whole = vec && i0 + V <= n;
+  const bool whole = VEC && i0 + V <= n;
   if (whole) {
 #pragma unroll
     for (int h = 0; h < V * (int)sizeof(T) / 32; ++h) {
@@ -166,33 +182,32 @@ __global__ void __launch_bounds__(256) k_frsz1_compress(const T* __restrict__ x,
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < V; ++k) xv[k] = i0 + k < n ? x[i0 + k] : (T)0;
+    for (int k = 0; k < V; ++k) xv[k] = i0 + k * STEP < n ? x[i0 + k * STEP] : (T)0;
   }
+  // the quantized value before value k: the thread's last one, or the lane's before
+  auto previous = [&](const auto(&q)[V], int k) {
+    using Q = std::decay_t<decltype(q[0])>;
+    if (VEC && k > 0) return q[k - 1];
+    Q p = __shfl_up_sync(0xFFFFFFFFu, q[VEC ? V - 1 : k], 1);
+    const Q first = VEC || k == 0 ? (Q)0 : __shfl_sync(0xFFFFFFFFu, q[VEC || k == 0 ? 0 : k - 1], 31);
+    return lane == 0 ? first : p;
+  };
   std::uint32_t w[V / 2];
-  {
+  if (__all_sync(0xFFFFFFFFu, legacy_in_range<T, V>(xv, inv))) {
     int q[V];
-    std::uint32_t off_hi = 0, off_lo = 0;
 #pragma unroll
-    for (int k = 0; k < V; ++k) q[k] = legacy_quantize_int<T>(xv[k], inv, off_hi, off_lo);
-    const bool off = off_hi != 0 || (off_lo >> 25) != 0;
-    int prev = __shfl_up_sync(0xFFFFFFFFu, q[V - 1], 1);
-    if (lane == 0) prev = 0;
-    if (!__any_sync(0xFFFFFFFFu, off)) {
+    for (int k = 0; k < V; ++k) q[k] = legacy_quantize_int<T>(xv[k], inv);
 #pragma unroll
-      for (int k = 0; k < V; k += 2)
-        w[k / 2] = pack_sat_s16(q[k] - (k == 0 ? prev : q[k - 1]), q[k + 1] - q[k]);
-    } else {
-      T f[V];
+    for (int k = 0; k < V; k += 2) w[k / 2] = pack_sat_s16(q[k] - previous(q, k), q[k + 1] - previous(q, k + 1));
+  } else {
+    T f[V];
 #pragma unroll
-      for (int k = 0; k < V; ++k) f[k] = legacy_quantize<T>(xv[k], inv);
-      T pf = __shfl_up_sync(0xFFFFFFFFu, f[V - 1], 1);
-      if (lane == 0) pf = (T)0;
+    for (int k = 0; k < V; ++k) f[k] = legacy_quantize<T>(xv[k], inv);
 #pragma unroll
-      for (int k = 0; k < V; k += 2) {
-        const std::int16_t a = legacy_saturate<T>(legacy_sub<T>(f[k], k == 0 ? pf : f[k - 1]));
-        const std::int16_t b = legacy_saturate<T>(legacy_sub<T>(f[k + 1], f[k]));
-        w[k / 2] = (std::uint16_t)a | ((std::uint32_t)(std::uint16_t)b << 16);
-      }
+    for (int k = 0; k < V; k += 2) {
+      const std::int16_t a = legacy_saturate<T>(legacy_sub<T>(f[k], previous(f, k)));
+      const std::int16_t b = legacy_saturate<T>(legacy_sub<T>(f[k + 1], previous(f, k + 1)));
+      w[k / 2] = (std::uint16_t)a | ((std::uint32_t)(std::uint16_t)b << 16);
     }
   }
   if (whole) {
@@ -205,7 +220,7 @@ __global__ void __launch_bounds__(256) k_frsz1_compress(const T* __restrict__ x,
   } else {
 #pragma unroll
     for (int k = 0; k < V; ++k)
-      if (i0 + k < n) out[i0 + k] = (std::int16_t)(w[k / 2] >> (16 * (k % 2)));
+      if (i0 + k * STEP < n) out[i0 + k * STEP] = (std::int16_t)(w[k / 2] >> (16 * (k % 2)));
   }
 }
 
@@ -473,8 +488,9 @@ int legacy_compress(double eps, const void* d_values, std::uint64_t n, void* d_o
                    reinterpret_cast<std::uintptr_t>(d_out) % 8 == 0;
   const std::uint64_t threads = (n + kComV - 1) / kComV;
   const unsigned grid = (unsigned)std::max<std::uint64_t>(1, (threads + 255) / 256);
-  launch(k_frsz1_compress<T>, grid, 256, 0, s, static_cast<const T*>(d_values), n, 1.0 / (eps * 2.0),
-         static_cast<std::int16_t*>(d_out), vec);
+  const auto kernel = vec ? k_frsz1_compress<T, true> : k_frsz1_compress<T, false>;
+  launch(kernel, grid, 256, 0, s, static_cast<const T*>(d_values), n, 1.0 / (eps * 2.0),
+         static_cast<std::int16_t*>(d_out));
   return cuda_status(cudaGetLastError(), "legacy compress launch");
 }
 
