@@ -247,8 +247,8 @@ __device__ __forceinline__ T legacy_step(std::int16_t q, double ebx2, T prev)
 // What bounds it: the chain of one value after the other (about 70 cycles in
 // fp32, 25 in fp64) against the warps the shared memory allows, and the length
 // of the runs in DRAM.  Measured on B200, 2^26 values, own differences, one
-// 16-value piece per block at a time (the kernel below) -> here: fp32 93.5 -> 72.8
-// us, fp64 153 -> 110.5 us; block 0's differences 67.3 -> 60.3 and 120 -> 101 us.
+// 16-value piece per block at a time (the kernel below) -> here: fp32 95 -> 69.9
+// us, fp64 153 -> 110 us; block 0's differences 68.5 -> 54.8 and 121 -> 98 us.
 // Runs of 32 bytes straight from registers took 115 / 171 us, of 128 bytes 75.8 /
 // 135 us, fp64 with 64 instead of 128 codes per stage 117 us, fp32 with 128
 // instead of 64 codes 82.5 us.
@@ -301,11 +301,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* g)
                : "memory");
 }
 
-template<class T, bool OWN, bool RND>
-__global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t* __restrict__ in, std::uint64_t n,
-                                                             double ebx2, T* __restrict__ y)
+// FULL: the CTA has 32 whole blocks.
+template<class T, bool OWN, bool RND, bool FULL>
+__device__ __forceinline__ void legacy_decompress_cta(const std::int16_t* __restrict__ in, std::uint64_t n,
+                                                      std::uint64_t v0, double ebx2, T* __restrict__ y,
+                                                      std::uint8_t* s_out, std::uint8_t* s_in)
 {
-  enter_in_stream_order();
   constexpr int VO = 64;                        // values per block and part
   constexpr int CS = sizeof(T) == 4 ? 64 : 128; // codes per block and stage
   constexpr int kOutBytes = VO * (int)sizeof(T);
@@ -313,12 +314,10 @@ __global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t*
   constexpr int CROW = 2 * CS + 16;                 // a block's row of codes
   constexpr int PV = 16 / (int)sizeof(T);           // values per 16 bytes
   constexpr int LPC = CS / 8, LPO = kOutBytes / 16; // threads per row of codes, of values
-  __shared__ __align__(16) std::uint8_t s_out[32 * kRowBytes];
-  __shared__ __align__(16) std::uint8_t s_in[OWN ? 2 * 32 * CROW : kLegacyBlock * 2];
   const int lane = threadIdx.x;
-  const std::uint64_t v0 = (std::uint64_t)blockIdx.x * (32 * kLegacyBlock); // the CTA's first value
-  const int full = (int)min((std::uint64_t)32, (n - v0) / kLegacyBlock);    // its whole blocks
-  const std::uint64_t g0 = v0 + (std::uint64_t)lane * kLegacyBlock;         // this thread's block
+  const int full = FULL ? 32 : (int)((n - v0) / kLegacyBlock);       // whole blocks
+  const int tail = FULL ? 0 : (int)(n - v0) - full * kLegacyBlock;   // values of the array's last, partial one
+  const std::uint64_t g0 = v0 + (std::uint64_t)lane * kLegacyBlock;  // this thread's block
   if constexpr (!OWN) { // block 0's codes, which every block adds
     for (int i = lane; i < kLegacyBlock; i += 32)
       reinterpret_cast<std::int16_t*>(s_in)[i] = (std::uint64_t)i < n ? in[i] : (std::int16_t)0;
@@ -330,10 +329,16 @@ __global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t*
     if constexpr (OWN) {
       if (stage < kLegacyBlock / CS) {
 #pragma unroll
-        for (int i = 0; i < LPC; ++i)
-          if ((32 / LPC) * i + lane / LPC < full)
-            cp_async16(s_src + (stage & 1) * (32 * CROW) + (32 / LPC) * i * CROW,
-                       src + stage * CS + (32 / LPC) * i * kLegacyBlock);
+        for (int i = 0; i < LPC; ++i) {
+          const int row = (32 / LPC) * i + lane / LPC;
+          std::uint8_t* d = s_src + (stage & 1) * (32 * CROW) + (32 / LPC) * i * CROW;
+          const std::int16_t* g = src + stage * CS + (32 / LPC) * i * kLegacyBlock;
+          if (FULL || row < full)
+            cp_async16(d, g);
+          else if (row == full) // in order with the copies: the partial block's codes one by one
+            for (int k = 0; k < 8 && stage * CS + (lane % LPC) * 8 + k < tail; ++k)
+              reinterpret_cast<std::int16_t*>(d)[k] = g[k];
+        }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     }
@@ -357,7 +362,7 @@ __global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t*
     for (int h = 0; h < VO; h += 8) {
       const uint4 c4 = *reinterpret_cast<const uint4*>(codes + h * 2);
       std::uint32_t w[4] = { c4.x, c4.y, c4.z, c4.w };
-      if (!OWN && h == 0 && part == 0 && lane < full)
+      if (!OWN && h == 0 && part == 0 && (FULL || g0 < n))
         w[0] = (w[0] & 0xFFFF0000u) | (std::uint16_t)in[g0]; // the block's own first value
 #pragma unroll
       for (int p = 0; p < 8; p += PV) {
@@ -386,20 +391,29 @@ __global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t*
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < LPO; ++i)
-      if ((32 / LPO) * i + lane / LPO < full)
+      if (FULL || (32 / LPO) * i + lane / LPO < full)
         __stcs(reinterpret_cast<uint4*>(dst + part * VO + (32 / LPO) * i * kLegacyBlock),
                *reinterpret_cast<const uint4*>(s_dst + (32 / LPO) * i * kRowBytes));
+    if constexpr (!FULL)
+      for (int k = part * VO + lane; k < min(tail, (part + 1) * VO); k += 32)
+        y[v0 + full * kLegacyBlock + k] = reinterpret_cast<const T*>(s_out + full * kRowBytes)[k - part * VO];
     __syncwarp(); // the part has left; its codes' buffer is free
   }
-  if (lane == full && g0 < n) { // the array's last, partial block
-    for (int i = 0; g0 + i < n; ++i) {
-      const std::int16_t q = OWN || i == 0 ? in[g0 + i] : reinterpret_cast<const std::int16_t*>(s_in)[OWN ? 0 : i];
-      const double t = __dmul_rn((double)q, ebx2);
-      acc.s = i == 0 ? t : __dadd_rn(t, acc.s);
-      acc.round_to_T();
-      y[g0 + i] = acc.value();
-    }
-  }
+}
+
+template<class T, bool OWN, bool RND>
+__global__ void __launch_bounds__(32) k_frsz1_decompress_vec(const std::int16_t* __restrict__ in, std::uint64_t n,
+                                                             double ebx2, T* __restrict__ y)
+{
+  enter_in_stream_order();
+  constexpr int CS = sizeof(T) == 4 ? 64 : 128; // codes per block and stage, as above
+  __shared__ __align__(16) std::uint8_t s_out[32 * (64 * sizeof(T) + 16)];
+  __shared__ __align__(16) std::uint8_t s_in[OWN ? 2 * 32 * (2 * CS + 16) : kLegacyBlock * 2];
+  const std::uint64_t v0 = (std::uint64_t)blockIdx.x * (32 * kLegacyBlock); // the CTA's first value
+  if (n - v0 >= 32 * kLegacyBlock)
+    legacy_decompress_cta<T, OWN, RND, true>(in, n, v0, ebx2, y, s_out, s_in);
+  else // whole blocks and the last, partial one side by side
+    legacy_decompress_cta<T, OWN, RND, false>(in, n, v0, ebx2, y, s_out, s_in);
 }
 
 // Blocks for pointers off the 32-byte layout: 64 blocks per CTA, values through
