@@ -24,7 +24,7 @@ def _after_pending_work(dst, src):
     dst.copy_(src, non_blocking=True)
 
 
-@pytest.mark.parametrize("n", [1000, 3_000_001])
+@pytest.mark.parametrize("n", [1000, 100_000, 3_000_001])
 @pytest.mark.parametrize("side", [False, True])
 @pytest.mark.parametrize("dtype,bits,E", [(np.float64, 32, 32), (np.float32, 13, 5)])
 def test_input_still_on_its_way(cuda, dtype, bits, E, n, side):
