@@ -557,7 +557,8 @@ template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
 __host__ __device__ constexpr bool decompress_straight()
 {
   constexpr bool F32 = sizeof(T) == 4;
-  if (MIS || HALF) return true;
+  if (HALF) return F32 || BITS < 64; // 2^24 / 2^26 values E 50: 64 bits 1.02 / 1.07 with the loop, 0.87 / 0.92 without
+  if (MIS) return true;
   if (GEN) return PAD || !(F32 ? BITS >= 8 && BITS <= 15 : BITS == 16); // fp32 12 bits E 24 1.03, 1.01 without
   if (PAD) return !F32 || BITS <= 24;                                   // fp32 29 bits E 8 1.06, 1.05
   if (ESM) return BITS <= (ESM == 4 ? 14 : 16) && (F32 || ESM == 1 || BITS > 8); // fp64 E 2 8 bits 1.01, 0.99
