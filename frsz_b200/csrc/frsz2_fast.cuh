@@ -582,8 +582,9 @@ __host__ __device__ constexpr bool decompress_straight()
 // warp's rows are consecutive (row = warp * RPW + rr), so a block lies in one
 // warp and its maximum needs no barrier.
 // FULL: the caller has seen that the tile is whole.
+// IMAX: block maxima by integer arithmetic (see launch_fast_one).
 template<class T, int BITS, int NT, int RPW_, bool PAD = false, int ESM = 0, bool MIS = false, bool GEN = false,
-         bool HALF = false, bool WCR = false, bool FULL = false>
+         bool HALF = false, bool WCR = false, bool FULL = false, bool IMAX = false>
 __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t tile, std::uint32_t* s_rmax,
                                                    std::uint32_t* s_stage, bool more_tiles = true,
                                                    std::uint32_t* s_gmax = nullptr, std::uint32_t mE = 0)
@@ -691,7 +692,7 @@ __device__ __forceinline__ void fast_compress_tile(const Job& j, std::uint64_t t
 #pragma unroll
     for (int rr = 0; rr < RPW; ++rr) {
       std::uint32_t m;
-      if constexpr (GEN && sizeof(T) == 8 && BITS > 32 && !Cfg::ALIGNED) {
+      if constexpr (IMAX || (GEN && sizeof(T) == 8 && BITS > 32 && !Cfg::ALIGNED)) {
         // the float maxima cost registers here (60 bits E 48: 0.91 of the integer maxima's speed)
         m = K::raw(u[rr][0]);
 #pragma unroll
@@ -1042,7 +1043,7 @@ __host__ __device__ constexpr int compress_ctas()
 }
 
 template<class T, int BITS, int NT = kNT, int RPW = 2, bool PAD = false, int ESM = 0, bool MIS = false,
-         bool GEN = false, bool HALF = false, bool WCR = false>
+         bool GEN = false, bool HALF = false, bool WCR = false, bool IMAX = false>
 __global__ void __launch_bounds__(NT, compress_ctas<T, BITS, PAD, ESM, MIS, GEN, HALF>()) k_compress_fast(Job j)
 {
   enter_in_stream_order();
@@ -1054,14 +1055,15 @@ __global__ void __launch_bounds__(NT, compress_ctas<T, BITS, PAD, ESM, MIS, GEN,
     const std::uint64_t tile = blockIdx.x;
     constexpr std::uint64_t TE = fast_cfg<T, BITS, NT, RPW, ESM>::TE;
     if (compress_splits<T, BITS, PAD, ESM, MIS, GEN, HALF>() && j.n - tile * TE >= TE)
-      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR, true>(j, tile, s_rmax, s_stage, false, s_gmax,
-                                                                              mE);
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR, true, IMAX>(j, tile, s_rmax, s_stage, false,
+                                                                                    s_gmax, mE);
     else
-      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR>(j, tile, s_rmax, s_stage, false, s_gmax, mE);
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR, false, IMAX>(j, tile, s_rmax, s_stage, false,
+                                                                                     s_gmax, mE);
   } else {
     for (std::uint64_t tile = blockIdx.x; tile < j.tiles; tile += gridDim.x)
-      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR>(j, tile, s_rmax, s_stage,
-                                                                          tile + gridDim.x < j.tiles, s_gmax, mE);
+      fast_compress_tile<T, BITS, NT, RPW, PAD, ESM, MIS, GEN, HALF, WCR, false, IMAX>(
+        j, tile, s_rmax, s_stage, tile + gridDim.x < j.tiles, s_gmax, mE);
   }
 }
 

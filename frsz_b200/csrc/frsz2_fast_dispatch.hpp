@@ -79,6 +79,17 @@ cudaError_t launch_fast_one(bool compress, const Job& j, cudaStream_t s, unsigne
     launch(k_compress_fast<T, BITS, kNT, 2, false, 0, false, false, false, true>, grid, kNT, 0, s, j);
     return cudaGetLastError();
   }
+  if constexpr (sizeof(T) == 4 && BITS == 32) {
+    // blocks that span more rows wait for one another at a barrier, and at this
+    // width the float maxima make that dearer (fraction of the copy bandwidth with
+    // integer / float maxima, 2^25 values: E 1024 1.00 / 0.93, E 4096 0.965 / 0.87; 2^27:
+    // 1.06 / 0.99, 1.03 / 0.93); without the barrier they are the better ones (E 32 at 2^27
+    // 1.05 / 1.07), and at 24 bits even
+    if (compress && j.E > 64 * fast_cfg<T, BITS>::P) {
+      launch(k_compress_fast<T, BITS, kNT, 2, false, 0, false, false, false, false, true>, grid, kNT, 0, s, j);
+      return cudaGetLastError();
+    }
+  }
   if (compress)
     launch(k_compress_fast<T, BITS>, grid, kNT, 0, s, j);
   else
