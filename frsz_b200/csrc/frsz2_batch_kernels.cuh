@@ -62,8 +62,7 @@ __host__ __device__ constexpr int batch_compress_ctas()
 // One CTA per tile of a class's concatenated tile list, the tile's array
 // read from a per-tile index (one 4-byte load): the launch shape of the
 // single-array kernels, which hardware CTA scheduling balances across SMs.
-// PADDED: some of the class's arrays have padded blocks (unaligned widths).  A
-// class without them takes the instance without their code.
+// PADDED: the instance that also takes padded blocks (unaligned widths).
 template<class T, int BITS, int NT, int RPW, bool COMPRESS, bool PADDED>
 __global__ void __launch_bounds__(NT, COMPRESS && !PADDED ? batch_compress_ctas<T, BITS>() : 0)
   k_batch_tiles(const BatchItem* __restrict__ items, const std::uint32_t* __restrict__ tile_item)
@@ -89,6 +88,18 @@ __global__ void __launch_bounds__(NT, COMPRESS && !PADDED ? batch_compress_ctas<
     fast_decompress_tile<T, BITS, NT, RPW>(j, lt);
 }
 
+// Whether a class without padded blocks has an instance without their code.
+// Compress always (it takes the cap above).  Decompress of fp64 above 16 bits: the
+// code's registers keep CTAs off the SM, which costs there and serves the narrow
+// widths (100 arrays of 2^20 values, time with their code / without: 17 bits 1.09, 18
+// bits 1.08, 20 bits 1.08, 52 bits 1.04, 38 and 46 bits 0.97; 5 to 7 bits 0.93, 13 to 15
+// bits 0.945; fp32 0.96 to 1.02, 1.00 over all widths).
+template<class T, int BITS>
+__host__ __device__ constexpr bool batch_unpadded(bool compress)
+{
+  return compress || (sizeof(T) == 8 && BITS > 16);
+}
+
 using batch_tiles_fn = cudaError_t (*)(bool compress, bool padded, const BatchItem* items,
                                        const std::uint32_t* tile_item, std::uint64_t tiles, cudaStream_t s);
 
@@ -97,18 +108,20 @@ cudaError_t launch_batch_tiles(bool compress, bool padded, const BatchItem* item
                                std::uint64_t tiles, cudaStream_t s)
 {
   const unsigned grid = (unsigned)tiles;
-  if constexpr (!fast_cfg<T, BITS, NT, RPW>::ALIGNED) {
-    if (padded) {
-      if (compress)
-        k_batch_tiles<T, BITS, NT, RPW, true, true><<<grid, NT, 0, s>>>(items, tile_item);
-      else
-        k_batch_tiles<T, BITS, NT, RPW, false, true><<<grid, NT, 0, s>>>(items, tile_item);
+  constexpr bool ALIGNED = fast_cfg<T, BITS, NT, RPW>::ALIGNED;
+  if constexpr (!ALIGNED) {
+    if (padded && compress) {
+      k_batch_tiles<T, BITS, NT, RPW, true, true><<<grid, NT, 0, s>>>(items, tile_item);
+      return cudaGetLastError();
+    }
+    if (!compress && (padded || !batch_unpadded<T, BITS>(false))) {
+      k_batch_tiles<T, BITS, NT, RPW, false, true><<<grid, NT, 0, s>>>(items, tile_item);
       return cudaGetLastError();
     }
   }
   if (compress)
     k_batch_tiles<T, BITS, NT, RPW, true, false><<<grid, NT, 0, s>>>(items, tile_item);
-  else
+  else if constexpr (ALIGNED || batch_unpadded<T, BITS>(false))
     k_batch_tiles<T, BITS, NT, RPW, false, false><<<grid, NT, 0, s>>>(items, tile_item);
   return cudaGetLastError();
 }
