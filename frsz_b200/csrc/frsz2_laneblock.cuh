@@ -372,7 +372,7 @@ cudaError_t launch_laneblock_f64(int bits, bool compress, const Job& j, cudaStre
 //     0.61 -> 0.66, 19 bits E 50 (17 KB) 0.67 -> 0.76, 31 bits E 50 (19 KB) 0.74 / 0.73, 41 bits
 //     E 50 (21 KB) 0.86 / 0.64
 // So the chunked kernels keep decompress where few warps fit beside that much
-// shared memory; above 128 values only the warp-per-block kernels are left.
+// shared memory.
 inline bool laneblock_eligible(const Job& j, std::size_t es, bool compress, const void* values, const void* words)
 {
   if (((reinterpret_cast<std::uintptr_t>(values) | reinterpret_cast<std::uintptr_t>(words)) & 15u) != 0) return false;
@@ -386,7 +386,20 @@ inline bool laneblock_eligible(const Job& j, std::size_t es, bool compress, cons
   const int any_length = compress ? 20 : j.bits > 32 ? 16 : es == 4 ? 24 : 20;
   if (j.n < enough && (j.E > any_length || (!compress && j.block_bytes % 32u == 0))) return false;
   const std::uint32_t smem = laneblock_smem(j, es, compress);
-  if (j.E > 128) return smem <= 48000u;
+  // above 128 values the warp-per-block kernels are the others.  Few warps fit beside
+  // that much shared memory, and compress needs more of them where it writes its image
+  // by bytes or half-words or reads its values one by one (time here over time there,
+  // compress, 2^25 fp32 / 2^24 fp64 values: bytes, fp32 4 bits E 250 36 KB 1.16, E 330 47
+  // KB 1.74, fp64 4 bits E 170 46 KB 1.57; half-words, fp32 14 bits E 250 46 KB 1.34, 13
+  // bits E 201 36 KB 0.61, fp64 12 bits E 150 46 KB 1.20, four values at a time 4 bits E
+  // 300 43 KB 0.77; words, fp32 16 bits E 230 44 KB 0.57, 23 bits E 201 44 KB 0.94, 25 bits
+  // 46 KB 1.09, images of a multiple of 32 bytes 19 bits E 201 42 KB 1.16; whole bytes, 8
+  // bits E 250 40 KB 0.67; decompress 0.3 to 1.06 throughout)
+  if (j.E > 128) {
+    const bool quads = laneblock_quads(j.E), words = j.block_bytes % 4u == 0, bytes = j.block_bytes % 2u != 0;
+    const bool any = !compress || j.bits == 8 || (words ? quads || j.block_bytes % 32u != 0 : quads && !bytes);
+    return smem <= (any ? 48000u : es == 8 ? (bytes ? 40500u : 43500u) : bytes ? 35500u : 41500u);
+  }
   if (compress) return smem <= (es == 4 ? 48000u : 32000u);
   // decompress: values of a multiple of 8 per block, or images of a multiple of 16
   // bytes, still meet four and more on a bank
