@@ -235,8 +235,16 @@ __global__ void __launch_bounds__(32) k_compress_laneblock(Job j)
       for (int i = 0; i < E; ++i) push_code(code(sv[i]));
     }
   };
-  if (__all_sync(0xFFFFFFFFu, plain)) {
-    const T scale = pow2<T>(BITS - 2 - be);
+  // a block of zeros, as that of a lane past the last one: no magnitude for either
+  // arithmetic, so it does not send the warp's other blocks to the slower one
+  bool zeros = km == 0;
+  if (sizeof(T) == 8 && zeros) { // km is the high words'
+    U low = 0;
+    for (int k = 0; k < E; ++k) low |= sv[k] << 1;
+    zeros = low == 0;
+  }
+  if (__all_sync(0xFFFFFFFFu, plain || zeros)) {
+    const T scale = pow2<T>(BITS - 2 - (zeros ? 0 : be));
     codes([&](U u) { return encode_plain<T, BITS>(u, scale); });
   } else {
     codes([&](U u) { return (C)to_code<T>(u, (std::int16_t)be, BITS); }); // exact for every block
