@@ -788,18 +788,19 @@ struct DotPlan
   unsigned grid;
 };
 
-// A warp walks up to 12 steps of 32 * NV positions (24 measured even), fewer
-// when that would leave fewer than three units for each of the 32 warps that an
+// A warp walks up to 12 steps of 32 * NV positions, 24 at 64 bits (dot of 100
+// vectors of 2^22 values: 64 bits 12 / 24 / 48 steps 621 / 602 / 619 us; 48 bits 12 / 24
+// steps 395 / 402), fewer when that would leave fewer than three units for each of the 32 warps that an
 // SM holds.  The workspace has room for max(8 per SM, n / 3072) sums per vector;
 // where short walks would need more, several warps of a CTA share a unit.
-bool dot_plan(int m, std::uint64_t n, int nv, int jb, DotPlan* p)
+bool dot_plan(int m, std::uint64_t n, int bits, int nv, int jb, DotPlan* p)
 {
   const std::uint64_t rows = std::max<std::uint64_t>((std::uint64_t)sm_count() * kMaxCtasPerSm, (n + kSub - 1) / kSub);
   const std::uint64_t step = 32 * (std::uint64_t)nv;
   const std::uint64_t groups = ((std::uint64_t)m + jb - 1) / jb;
   const std::uint64_t steps = (n + step - 1) / step;
   const std::uint64_t warps = (std::uint64_t)sm_count() * 32 * 3;
-  std::uint64_t k = std::min<std::uint64_t>(12, std::max<std::uint64_t>(1, (steps * groups + warps - 1) / warps));
+  std::uint64_t k = std::min<std::uint64_t>(bits > 48 ? 24 : 12, std::max<std::uint64_t>(1, (steps * groups + warps - 1) / warps));
   const std::uint64_t least = (steps + rows - 1) / rows; // steps per slice that the workspace asks for
   int lq = 0;
   while (lq < 3 && (k << lq) < least) ++lq;
@@ -818,7 +819,7 @@ int launch_dot(const BasisParams& bp, int m, const BasisGeo& g, const double* w,
                cudaStream_t s)
 {
   DotPlan p;
-  if (!dot_plan(m, g.n, NV, JB, &p)) return set_error(FRSZ2_EFAIL, "basis vectors too long");
+  if (!dot_plan(m, g.n, BITS, NV, JB, &p)) return set_error(FRSZ2_EFAIL, "basis vectors too long");
   auto* rows = reinterpret_cast<double*>(static_cast<std::uint8_t*>(workspace) + 256);
   launch(k_basis_dot<BITS, NV, JB>, p.grid, kKT, 0, s, bp, m, g, w, p.ns, p.groups, p.S, p.lq, rows);
   if (int rc = cuda_status(cudaGetLastError(), "basis dot launch")) return rc;
