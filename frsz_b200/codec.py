@@ -60,20 +60,22 @@ def exponent_size(dtype, bits: int, block_size: int, n: int) -> int:
     return out.value
 
 
+_WORD_BYTES = tuple(word_bits(bits) // 8 for bits in range(65))
+
+
 def _size(code: int, bits: int, block_size: int, n: int) -> int:
     """compressed_size without a call into the library, for every launch's
     check of its buffer.  Python integers only: those of numpy and torch would
     wrap at their own width, so they go to the library, and so does what is out
     of range, which it names."""
-    if not (type(bits) is type(block_size) is type(n) is int
-            and 4 <= bits <= (64 if code else 32) and 1 <= block_size <= 65536 and 0 <= n < 1 << 48):
-        out = ctypes.c_uint64()
-        check(lib().frsz2_compressed_size(code, bits, block_size, n, ctypes.byref(out)))
-        return out.value
-    w = 1 if bits <= 8 else 2 if bits <= 16 else 4 if bits <= 32 else 8
-    nb = -(-n // block_size)
-    e = nb * w
-    return e + 256 - e % 256 + nb * (-(-block_size * bits // (8 * w)) * w)
+    if (type(bits) is type(block_size) is type(n) is int
+            and 3 < bits < (65 if code else 33) and 0 < block_size < 65537 and -1 < n < 1 << 48):
+        w = _WORD_BYTES[bits]
+        nb = (n - 1) // block_size + 1
+        return (nb * w | 255) + 1 + ((block_size * bits - 1) // (8 * w) + 1) * w * nb
+    out = ctypes.c_uint64()
+    check(lib().frsz2_compressed_size(code, bits, block_size, n, ctypes.byref(out)))
+    return out.value
 
 
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)

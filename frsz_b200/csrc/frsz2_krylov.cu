@@ -455,46 +455,28 @@ __device__ __noinline__ void rest_of_axpy(const std::uint8_t* const* bufs, int l
   for (int k = 0; k < NV; ++k) y[k] = acc[k];
 }
 
-// Sums of N (a power of two up to 32) values over the warp in a fixed order:
-// each exchange halves the values a lane carries, so N values cost N - 1 +
-// log2(32 / N) exchanges instead of 5 N.  Returns the sum of value
-// (lane * N) / 32.
+// Sums of two or four values over the warp in a fixed order: each exchange halves
+// the values a lane carries, so N values cost N - 1 + log2(32 / N) exchanges
+// instead of 5 N.  Returns value (lane * N) / 32 summed over the lanes that share
+// this one's lower bits; the caller adds those up.
 template<int N>
 __device__ __forceinline__ double warp_sums(double (&a)[N])
 {
+  static_assert(N == 2 || N == 4, "two or four values");
   const int lane = threadIdx.x & 31;
-  if constexpr (N == 1) {
-    return a[0];
+  const bool up = (lane & 16) != 0;
+  double b[N / 2];
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const double send = up ? a[i] : a[i + N / 2];
+    b[i] = (up ? a[i + N / 2] : a[i]) + __shfl_xor_sync(0xFFFFFFFFu, send, 16);
+  }
+  if constexpr (N == 2) {
+    return b[0];
   } else {
-    constexpr int H = N / 2;
-    double b[H];
-#pragma unroll
-    for (int i = 0; i < H; ++i) {
-      // the distance between the two halves of the lanes at this level
-      const bool up = (lane & 16) != 0;
-      const double send = up ? a[i] : a[i + H];
-      b[i] = (up ? a[i + H] : a[i]) + __shfl_xor_sync(0xFFFFFFFFu, send, 16);
-    }
-    if constexpr (H == 1) {
-      return b[0];
-    } else {
-      constexpr int Q = H / 2;
-      double c[Q];
-#pragma unroll
-      for (int i = 0; i < Q; ++i) {
-        const bool up = (lane & 8) != 0;
-        const double send = up ? b[i] : b[i + Q];
-        c[i] = (up ? b[i + Q] : b[i]) + __shfl_xor_sync(0xFFFFFFFFu, send, 8);
-      }
-      if constexpr (Q == 1) {
-        return c[0];
-      } else {
-        static_assert(Q == 2, "at most eight values");
-        const bool up = (lane & 4) != 0;
-        const double send = up ? c[0] : c[1];
-        return (up ? c[1] : c[0]) + __shfl_xor_sync(0xFFFFFFFFu, send, 4);
-      }
-    }
+    const bool up2 = (lane & 8) != 0;
+    const double send = up2 ? b[0] : b[1];
+    return (up2 ? b[1] : b[0]) + __shfl_xor_sync(0xFFFFFFFFu, send, 8);
   }
 }
 
@@ -513,7 +495,6 @@ __global__ void __launch_bounds__(kKT, dot_ctas(BITS, NV, JB))
               unsigned groups, unsigned S, int lq, double* __restrict__ partials)
 {
   enter_in_stream_order();
-  static_assert((JB & (JB - 1)) == 0 && JB <= 8, "warp_sums");
   constexpr int Wb = fast_cfg<double, BITS>::W / 8;
   __shared__ double s_sum[kKW][JB];
   const int lane = threadIdx.x & 31;
