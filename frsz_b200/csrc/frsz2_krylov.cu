@@ -65,10 +65,11 @@ __host__ __device__ constexpr int dot_ctas(int bits, int nv, int jb)
 // axpy over 2..12 x 2..4 (us): 16 bits 6 x 3 170, 5 x 3 179, 3 x 4 182, 4 x 3 230;
 // 21 bits 5 x 3 67.1, 4 x 3 67.8; 24 bits 3 x 4 62.0, 4 x 3 65.3; 32 bits 4 x 3
 // 262, 3 x 4 265, 6 x 3 366 (spills); 48 bits 5 x 3 103, 4 x 3 118; 64 bits 5 x 3
-// 132, 4 x 3 133; four values per lane, 32 bits 6 x 4 45.7, 5 x 3 49.6.
+// 132, 4 x 3 133; four values per lane, 100 vectors of 2^20, 6 x 4 / 5 x 4: 16 bits
+// 63.8 / 57.0, 21 bits 83.6 / 78.0, 24 bits 65.6 / 63.9, 32 bits 68.2 / 72.4.
 __host__ __device__ constexpr int axpy_jb(int bits, int nv)
 {
-  if (nv == 4 && bits <= 32) return 6;
+  if (nv == 4 && bits <= 32) return bits == 32 ? 6 : 5;
   return bits == 16 ? 6 : bits == 24 ? 3 : bits == 32 ? 4 : 5;
 }
 __host__ __device__ constexpr int axpy_ctas(int bits, int nv)
