@@ -515,7 +515,8 @@ __device__ __forceinline__ void load_lane_exps(const std::uint8_t* p, std::int64
 
 // Whether a whole tile of compress is coded by an instance of its own, without the
 // partial tile's bounds: narrow widths, blocks below a lane, and values off the
-// 32-byte layout, where instructions bound the kernel.  Of the copy bandwidth, one
+// 32-byte layout, where instructions bound the kernel.  The lines are where the
+// measurements turn, one sweep over the widths at E 32 and a few other sizes.  Of the copy bandwidth, one
 // instance -> two, both without the loop (below): fp32 6 bits E 128 1.056 -> 1.078,
 // E 1024 0.92 -> 1.00, E 2 at 8 bits 0.80 -> 0.88, off by one 8 bits 0.98 -> 1.02; fp64 13 bits
 // E 512 1.03 -> 1.07, E 1 at 16 bits 0.99 -> 1.06.  Wider, the two cost registers (fp64
@@ -534,14 +535,17 @@ __host__ __device__ constexpr bool compress_splits()
 
 // Whether a CTA takes its one tile (the grid is the tiles) or keeps a loop over
 // tiles that never comes round.  Without the loop's variables and branches there
-// are registers and instructions to spare: of the copy bandwidth, loop -> none,
-// compress fp32 6 bits E 128 0.94 -> 1.06, 9 bits E 64 0.99 -> 1.08, E 24 8 bits 0.94 ->
-// 1.03, off by one 12 bits 0.94 -> 1.02, padded 29 bits E 8 0.90 -> 0.95, fp64 9 bits E
-// 64 0.97 -> 1.08, 47 bits 0.98 -> 1.02; decompress fp32 off by one 16 bits 0.92 -> 1.03,
-// E 1 at 12 bits 0.75 -> 1.03, E 20 at 12 bits 0.91 -> 1.01, fp64 6 bits 0.91 -> 1.01,
-// padded 21 bits 0.93 -> 1.02.  The loop stays where more CTAs at once move less than
-// fewer (DRAM pages): compress fp32 16 bits 1.07 -> 1.06, 32 bits 1.065 -> 1.04, fp64 24
-// bits 1.09 -> 1.075; decompress fp32 13 bits 1.04 -> 1.00, fp64 29 bits 1.00 -> 0.97.
+// are registers and instructions to spare, and most instances gain: of the copy
+// bandwidth, loop -> none, compress fp32 6 bits E 128 0.94 -> 1.06, 9 bits E 64 0.99 ->
+// 1.08, E 24 8 bits 0.94 -> 1.03, off by one 12 bits 0.94 -> 1.02, padded 29 bits E 8
+// 0.90 -> 0.95, fp64 9 bits E 64 0.97 -> 1.08, 47 bits 0.98 -> 1.02; decompress fp32 off
+// by one 16 bits 0.92 -> 1.03, E 1 at 12 bits 0.75 -> 1.03, E 20 at 12 bits 0.91 -> 1.01,
+// fp64 6 bits 0.91 -> 1.01, padded 21 bits 0.93 -> 1.02.  The loop stays where it
+// measured faster, mostly by 1 to 4 %: compress fp32 16 bits 1.07 -> 1.06, 32 bits 1.065
+// -> 1.04, fp64 24 bits 1.09 -> 1.075; decompress fp32 13 bits 1.04 -> 1.00, fp64 29
+// bits 1.00 -> 0.97.  What tells these widths from their neighbours was not found
+// (more tiles in flight at once may open more DRAM pages), so the lists below are
+// measurements, each width's own, and a change to the tile's code asks for them again.
 // Every width was measured at E 32, most at E 256, fp32 2^27 / fp64 2^26 values.
 template<class T, int BITS, bool PAD, int ESM, bool MIS, bool GEN, bool HALF>
 __host__ __device__ constexpr bool compress_straight()

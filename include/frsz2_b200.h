@@ -89,9 +89,11 @@ int frsz2_decompress(int dtype, int bits, int block_size, const void* d_compress
 
 /* Host buffers: the same codec with the host<->device copies inside the call
  * (pinned memory recommended; pageable works).  Synchronous: returns when the
- * result is in host memory.  This is the drop-in for the reference's host-side
- * compress_cpu_impl / decompress_cpu_impl calls.  Pinned buffers transfer
- * directly.  Ordinary memory goes through pinned slots (up to 48 MiB pinned and
+ * result is in host memory, and in order: after all that `stream` holds, so an
+ * input may still be on its way there.  This is the drop-in for the reference's
+ * host-side compress_cpu_impl / decompress_cpu_impl calls.  Buffers pinned on both
+ * sides transfer directly, and so do those pinned on one side between 64 KiB and 8
+ * MiB of values.  Ordinary memory goes through pinned slots (up to 48 MiB pinned and
  * 48 MiB of device memory per device, kept) by up to 12 threads that end with
  * the call, three quarters of the host's cores at most. */
 int frsz2_compress_host(int dtype, int bits, int block_size, const void* h_values, uint64_t n, void* h_compressed,
